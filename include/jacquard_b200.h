@@ -145,6 +145,53 @@ int jq_plain_prepare(const size_t *blocks_start, const uint32_t *blocks_data, si
                      size_t num_major_stages, uint32_t *stage_depth_base, uint8_t *stage_depth,
                      size_t depth_capacity, size_t *num_stages, void *stream);
 
+/* Gate-list plan of a script for one-stream runs (no counterpart in the
+ * reference).  jq_plain_plan_build resolves every partition to the state
+ * words and bits it reads, its live gates by logic level and its writeout
+ * references, into a caller-owned device workspace (16-byte aligned,
+ * jq_plain_plan_words words; it must outlive the plan, and only its first
+ * used_words words are needed afterwards), and synchronizes `stream`.
+ * state_words: the value words of a snapshot (reg_io_state_size; a larger
+ * number is fine).  target_items: work items per major stage that
+ * partitions are split towards (0 = default; 0xffffffff = default, and never
+ * the mirrored form).  `supported` is 0 for a script
+ * that the plan does not represent: one whose partitions read writeout slots
+ * that nothing in the partition writes, or words of their own major stage,
+ * or that exceed its limits; jq_simulate runs those. */
+typedef struct {
+  size_t num_blocks, num_major_stages;
+  uint32_t supported;                   /* 0: not represented, run jq_simulate */
+  uint32_t max_blob, max_slots, max_gw; /* largest item */
+  uint32_t stage_item[33];              /* first item of each major stage */
+  uint32_t widest, nbuf;                /* most items of a stage, blob buffers */
+  /* form that keeps the snapshot in the shared memory of one cluster */
+  uint32_t mirrored, rio, xoff, n_unwritten, stage_words[32];
+  const uint32_t *unwritten;
+  size_t exchange_words; /* of a launch's exchange buffer (device, 16-byte aligned) */
+  size_t used_words;
+  const uint32_t *blob;                 /* device, inside the workspace */
+  const unsigned long long *item_off;
+  const uint32_t *item_words;
+} jq_plain_plan;
+size_t jq_plain_plan_words(size_t blocks_data_len, size_t num_blocks, size_t num_major_stages,
+                           size_t state_words);
+int jq_plain_plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t num_blocks,
+                        size_t num_major_stages, size_t state_words, uint32_t target_items,
+                        uint32_t *workspace, size_t workspace_words, jq_plain_plan *plan,
+                        void *stream);
+
+/* jq_simulate on a plan of the same script: the same snapshots, SRAM
+ * contents and events (asynchronous, status by jq_sim_status).  exchange:
+ * device buffer of exchange_words words (NULL when 0), cleared by the launch
+ * and used until it ends, so launches that may overlap need their own.
+ * state_size must cover the plan's words (and X words).  Setup/hold
+ * checks and arrivals take each state word's arrival from two tables, as
+ * jq_simulate_batched does (arrival_first, arrival_steady: required with
+ * constraints or an arrival section, else unused). */
+int jq_simulate_planned(const jq_sim_args *a, const jq_plain_plan *plan,
+                        const uint32_t *arrival_first, const uint32_t *arrival_steady,
+                        uint32_t *exchange);
+
 /* Largest grid the plain interpreter can keep co-resident on `device`. */
 int jq_max_blocks(int device, size_t *max_blocks);
 

@@ -340,25 +340,8 @@ class BatchedSim:
 
 def arrival_tables(script, device="cuda", stream=None):
     """The u16 arrival of every state word in the first cycle of a launch
-    and in later cycles (int32 device tensors of reg_io_state_size words):
-    the arrival sections of snapshots 1 and 2 of a two-cycle run of the
-    plain interpreter on the same script.  Arrivals follow from the script's
-    delays and each block's execution order, not from the stimulus, so an
-    all-zero state serves."""
-    rio = script.reg_io_state_size
-    eff = rio * (2 if script.xprop_enabled else 1) + rio  # + arrival section
-    ds = sim.DeviceScript(script, device)
-    st = torch.zeros(3 * eff, dtype=torch.int32, device=device)
-    n_sram = max(1, script.sram_storage_size)
-    sram = torch.zeros(n_sram, dtype=torch.int32, device=device)
-    sram_x = torch.zeros(n_sram, dtype=torch.int32, device=device)
-    off = eff - rio
-    sim.simulate(ds, st, 2, eff, sram, sram_x, arrival_state_offset=off, stream=stream)
-    rc = sim.status(stream)
-    if rc:
-        raise RuntimeError("arrival tables: " + sim.lib().jq_strerror(rc).decode())
-    snaps = st.view(3, eff)
-    return snaps[1, off:].clone(), snaps[2, off:].clone()
+    and in later cycles (sim.arrival_tables)."""
+    return sim.arrival_tables(sim.DeviceScript(script, device), stream)
 
 
 class Timing:

@@ -25,6 +25,19 @@ class SimArgs(ctypes.Structure):
                 ("stage_depth", vp), ("stage_depth_base", vp)]
 
 
+class PlainPlan(ctypes.Structure):
+    _fields_ = [("num_blocks", ctypes.c_size_t), ("num_major_stages", ctypes.c_size_t),
+                ("supported", ctypes.c_uint32), ("max_blob", ctypes.c_uint32),
+                ("max_slots", ctypes.c_uint32), ("max_gw", ctypes.c_uint32),
+                ("stage_item", ctypes.c_uint32 * 33), ("widest", ctypes.c_uint32),
+                ("nbuf", ctypes.c_uint32), ("mirrored", ctypes.c_uint32), ("rio", ctypes.c_uint32),
+                ("xoff", ctypes.c_uint32), ("n_unwritten", ctypes.c_uint32),
+                ("stage_words", ctypes.c_uint32 * 32), ("unwritten", vp),
+                ("exchange_words", ctypes.c_size_t), ("used_words", ctypes.c_size_t),
+                ("blob", vp), ("item_off", vp), ("item_words", vp)]
+
+
+PLAN_NO_MIRROR = 0xFFFFFFFF
 EVENT_WORDS = 8
 EVENT_HEADER_WORDS = 4
 
@@ -41,6 +54,14 @@ def lib():
         L.jq_plain_prepare.restype = ctypes.c_int
         L.jq_plain_prepare.argtypes = [vp, vp, ctypes.c_size_t, ctypes.c_size_t, vp, vp,
                                        ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t), vp]
+        L.jq_plain_plan_words.restype = ctypes.c_size_t
+        L.jq_plain_plan_words.argtypes = [ctypes.c_size_t] * 4
+        L.jq_plain_plan_build.restype = ctypes.c_int
+        L.jq_plain_plan_build.argtypes = [vp, vp, ctypes.c_size_t, ctypes.c_size_t, ctypes.c_size_t,
+                                          ctypes.c_uint32, vp, ctypes.c_size_t,
+                                          ctypes.POINTER(PlainPlan), vp]
+        L.jq_simulate_planned.restype = ctypes.c_int
+        L.jq_simulate_planned.argtypes = [ctypes.POINTER(SimArgs), ctypes.POINTER(PlainPlan), vp, vp, vp]
         L.jq_strerror.restype = ctypes.c_char_p
         L.jq_strerror.argtypes = [ctypes.c_int]
         sz, u32p, i32 = ctypes.c_size_t, vp, ctypes.c_int32
@@ -72,6 +93,60 @@ class DeviceScript:
             np.ascontiguousarray(script.blocks_start, dtype=np.uint64).view(np.int64)).to(device)
         self.blocks_data = u32_to_dev(script.blocks_data, device)
         self._depth = None
+        self._plan = None
+        self._arrivals = None
+        self._exchange = {}
+
+    def plan(self, target_items=0):
+        """The script's gate-list plan (jq_plain_plan_build), or None when the
+        script is not one it represents; built on first use.  target_items is
+        jq_plain_plan_build's (0: its default, PLAN_NO_MIRROR: never the form
+        that keeps the state in shared memory)."""
+        if self._plan is None:
+            L = lib()
+            dev = self.blocks_data.device
+            rio = self.script.reg_io_state_size
+            n = L.jq_plain_plan_words(self.blocks_data.numel(), self.num_blocks,
+                                      self.num_major_stages, rio)
+            ws = torch.empty(n, dtype=torch.int32, device=dev)
+            p = PlainPlan()
+            rc = L.jq_plain_plan_build(self.blocks_start.data_ptr(), self.blocks_data.data_ptr(),
+                                       self.num_blocks, self.num_major_stages, rio, target_items,
+                                       ws.data_ptr(), n, ctypes.byref(p), torch.cuda.current_stream(dev).cuda_stream)
+            if rc:
+                raise RuntimeError("jq_plain_plan_build: " + L.jq_strerror(rc).decode())
+            if p.supported:  # keep the used part only
+                used = ws[:p.used_words].clone()
+                for f in ("blob", "item_off", "item_words", "unwritten"):
+                    setattr(p, f, getattr(p, f) - ws.data_ptr() + used.data_ptr())
+                torch.cuda.current_stream(dev).synchronize()
+                self._plan = (p, used)
+            else:
+                self._plan = (None, None)
+        return self._plan[0]
+
+    def exchange(self, stream=None):
+        """Device pointer of the exchange buffer for planned launches on this
+        stream (one per stream, allocated on it, so launches on two streams
+        may overlap; kept with the script), or None when the plan needs none."""
+        n = self._plan[0].exchange_words
+        if not n:
+            return None
+        if stream is None:
+            stream = torch.cuda.current_stream(self.blocks_data.device)
+        buf = self._exchange.get(stream.cuda_stream)
+        if buf is None:
+            with torch.cuda.stream(stream):
+                buf = torch.empty(n, dtype=torch.int32, device=self.blocks_data.device)
+            self._exchange[stream.cuda_stream] = buf
+        return buf.data_ptr()
+
+    def arrivals(self):
+        """(first cycle's, later cycles') u16 arrival of every state word, in
+        int32 device tensors; computed on first use."""
+        if self._arrivals is None:
+            self._arrivals = arrival_tables(self)
+        return self._arrivals
 
     def depth(self, stream=None):
         """(stage depth codes, per-entry base) on the device
@@ -105,12 +180,21 @@ def max_blocks(device=0):
     return n.value
 
 
+def _capturing(stream):
+    if stream is None:
+        return torch.cuda.is_current_stream_capturing()
+    with torch.cuda.stream(stream):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=None,
              events=None, event_capacity=0, arrival_state_offset=0, first_cycle=0,
-             stream=None, barrier_timeout_cycles=0, skip_dead_levels=True):
+             stream=None, barrier_timeout_cycles=0, skip_dead_levels=True, planned=True):
     """Launch the plain interpreter (asynchronous).  All tensors on device.
     skip_dead_levels: pass the script's stage-depth tables, so tree levels
-    whose outputs nothing reads are skipped (False runs every level)."""
+    whose outputs nothing reads are skipped (False runs every level).
+    planned: run the script's gate-list plan when it has one and the barrier
+    wait is not bounded by the caller (skip_dead_levels only)."""
     a = SimArgs(ds.num_blocks, ds.num_major_stages, ds.blocks_start.data_ptr(),
                 ds.blocks_data.data_ptr(), sram.data_ptr(),
                 sram_x.data_ptr() if sram_x is not None else None, num_cycles, state_size,
@@ -118,6 +202,21 @@ def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=
                 events.data_ptr() if events is not None else None, event_capacity,
                 arrival_state_offset, first_cycle, barrier_timeout_cycles,
                 stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream)
+    if skip_dead_levels and planned and not barrier_timeout_cycles:
+        tracked = bool(arrival_state_offset) or constraints is not None
+        # the plan and the arrival tables are made on first use, which a
+        # stream capture cannot record: such a call runs the script's own form
+        ready = ds._plan is not None and (ds._arrivals is not None or not tracked)
+        plan = ds.plan() if ready or not _capturing(stream) else None
+        if plan is not None:
+            first = steady = None
+            if tracked:
+                first, steady = (t.data_ptr() for t in ds.arrivals())
+            rc = lib().jq_simulate_planned(ctypes.byref(a), ctypes.byref(plan), first, steady,
+                                           ds.exchange(stream))
+            if rc:
+                raise RuntimeError("jq_simulate: " + lib().jq_strerror(rc).decode())
+            return
     if skip_dead_levels:
         depth, base = ds.depth(stream)
         a.stage_depth = depth.data_ptr()
@@ -125,6 +224,29 @@ def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=
     rc = lib().jq_simulate(ctypes.byref(a))
     if rc:
         raise RuntimeError("jq_simulate: " + lib().jq_strerror(rc).decode())
+
+
+def arrival_tables(ds, stream=None):
+    """The u16 arrival of every state word in the first cycle of a launch
+    and in later cycles (int32 device tensors of reg_io_state_size words):
+    the arrival sections of snapshots 1 and 2 of a two-cycle run of the
+    script itself.  Arrivals follow from the script's delays and each block's
+    execution order, not from the stimulus, so an all-zero state serves."""
+    s = ds.script
+    rio = s.reg_io_state_size
+    eff = rio * (2 if s.xprop_enabled else 1) + rio  # + arrival section
+    dev = ds.blocks_data.device
+    st = torch.zeros(3 * eff, dtype=torch.int32, device=dev)
+    n_sram = max(1, s.sram_storage_size)
+    sram = torch.zeros(n_sram, dtype=torch.int32, device=dev)
+    sram_x = torch.zeros(n_sram, dtype=torch.int32, device=dev)
+    off = eff - rio
+    simulate(ds, st, 2, eff, sram, sram_x, arrival_state_offset=off, stream=stream, planned=False)
+    rc = status(stream)
+    if rc:
+        raise RuntimeError("arrival tables: " + lib().jq_strerror(rc).decode())
+    snaps = st.view(3, eff)
+    return snaps[1, off:].clone(), snaps[2, off:].clone()
 
 
 def status(stream=None):
