@@ -55,7 +55,7 @@ WORKLOADS = {
 
 
 PROFILE_BATCHED = os.path.join(HERE, "profiles", "batched_kernel_soc2M_xprop.md")
-KERNEL_SRC = os.path.join(HERE, "jacquard_b200", "csrc", "sim_batched.cu")
+KERNEL_SRC = os.path.join(HERE, "jacquard_b200", "csrc", "batched_plan.cuh")
 
 
 def kernel_code_hash(path=KERNEL_SRC):
@@ -317,11 +317,14 @@ def algorithmic_bytes_per_cycle(s, streams=1, arrivals=False, bit_sliced=False):
 
 def prepared_script_bytes(B):
     """Script bytes the batched kernel must stream per simulated cycle, once
-    per partition (all streams share them): the metadata (1 KB), a 4-byte
+    for all streams: the blobs of the gate-list plan's items, or without a
+    plan, per partition, the metadata (1 KB), a 4-byte
     source entry per global-read slot it loads, and the copied part of each
     chunk of the prepared script (the used head of a compact chunk, the whole
     20 KB chunk otherwise).  The rest of FlattenedScriptV1's fixed-size
     chunks is padding the kernel never reads."""
+    if B.plan is not None:
+        return 4 * B.plan_words()
     bd = B.prepared.cpu().numpy().view(np.uint32)
     bs = np.asarray(B.script.blocks_start, np.int64)
     total = 0

@@ -317,6 +317,42 @@ int jq_batched_prepare(const size_t *blocks_start, const uint32_t *blocks_data,
                        size_t num_partitions, uint32_t *out, uint32_t *part_base,
                        uint32_t *gr_sources, void *stream);
 int jq_simulate_batched(const jq_batch_args *a);
+
+/* Gate-list plan of a script (the original, not the prepared one) for batched
+ * runs of `lanes` lane words in items of lanes_per_item (1 or 2 in layouts 0
+ * and 1, 8 in layouts 2 and 3), in a caller-owned device workspace as for
+ * jq_plain_plan_build; synchronizes `stream`.  Layout 3 (lane octets without
+ * X: word ((l >> 3) * signals + s) * 8 + (l & 7), lanes a multiple of 8) is
+ * one that only planned launches run.  `supported` is 0 for scripts it does
+ * not represent (see jq_plain_plan_build) and for items whose slots do not fit
+ * the shared memory.  state_words: the value words of a snapshot, exactly
+ * (the X offset of every X-capable partition). */
+typedef struct {
+  size_t num_major_stages, num_partitions;
+  uint32_t lanes, lanes_per_item;
+  int32_t x_interleaved;
+  uint32_t with_x, supported;
+  uint32_t max_blob, max_slots, nbuf; /* largest item, blob buffers */
+  uint32_t widest, stage_item[33];    /* most items of a stage, first of each */
+  size_t used_words;
+  const uint32_t *blob;               /* device, inside the workspace */
+  const unsigned long long *item_off;
+  const uint32_t *item_words;
+} jq_batched_plan;
+size_t jq_batched_plan_words(size_t blocks_data_len, size_t num_blocks, size_t num_major_stages,
+                             size_t state_words);
+int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_data,
+                          size_t num_blocks, size_t num_major_stages, size_t state_words,
+                          uint32_t lanes, uint32_t lanes_per_item, int32_t x_interleaved,
+                          uint32_t *workspace, size_t workspace_words, jq_batched_plan *plan,
+                          void *stream);
+/* jq_simulate_batched on a plan: the same states, outputs, SRAM contents and
+ * events.  Of the arguments it does not use blocks_start, blocks_data,
+ * num_blocks, part_base, gr_sources, wo_slots, block_list(_start) and
+ * lanes_per_item; part_cycles counts the items of a split partition
+ * together. */
+int jq_simulate_batched_planned(const jq_batch_args *a, const jq_batched_plan *plan);
+
 /* Words of one batched state buffer. */
 size_t jq_batched_state_words(uint32_t lanes, size_t signals);
 /* Lane-major [lanes][signals] (device) <-> batched state layout (device),

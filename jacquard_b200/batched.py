@@ -33,6 +33,17 @@ class BatchArgs(ctypes.Structure):
                 ("events", vp), ("event_capacity", ctypes.c_uint32), ("first_cycle", ctypes.c_uint32)]
 
 
+class BatchedPlan(ctypes.Structure):
+    _fields_ = [("num_major_stages", ctypes.c_size_t), ("num_partitions", ctypes.c_size_t),
+                ("lanes", ctypes.c_uint32),
+                ("lanes_per_item", ctypes.c_uint32), ("x_interleaved", ctypes.c_int32),
+                ("with_x", ctypes.c_uint32), ("supported", ctypes.c_uint32),
+                ("max_blob", ctypes.c_uint32), ("max_slots", ctypes.c_uint32),
+                ("nbuf", ctypes.c_uint32), ("widest", ctypes.c_uint32),
+                ("stage_item", ctypes.c_uint32 * 33), ("used_words", ctypes.c_size_t),
+                ("blob", vp), ("item_off", vp), ("item_words", vp)]
+
+
 def lib():
     L = load("libjacquard_b200.so")
     if not getattr(L, "_jq_batched_typed", False):
@@ -56,6 +67,14 @@ def lib():
         L.jq_batched_oct_capacity.argtypes = [ctypes.POINTER(ctypes.c_uint32)]
         L.jq_batched_slot_need.restype = ctypes.c_int
         L.jq_batched_slot_need.argtypes = [vp, vp, ctypes.c_size_t, ctypes.c_size_t, vp, vp]
+        L.jq_batched_plan_words.restype = ctypes.c_size_t
+        L.jq_batched_plan_words.argtypes = [ctypes.c_size_t] * 4
+        L.jq_batched_plan_build.restype = ctypes.c_int
+        L.jq_batched_plan_build.argtypes = [vp, vp] + [ctypes.c_size_t] * 3 + \
+            [ctypes.c_uint32, ctypes.c_uint32, ctypes.c_int32, vp, ctypes.c_size_t,
+             ctypes.POINTER(BatchedPlan), vp]
+        L.jq_simulate_batched_planned.restype = ctypes.c_int
+        L.jq_simulate_batched_planned.argtypes = [ctypes.POINTER(BatchArgs), ctypes.POINTER(BatchedPlan)]
         L._jq_batched_typed = True
     return L
 
@@ -179,31 +198,16 @@ class BatchedSim:
     """Script + buffers on the device for `lanes` lane words (32*lanes streams)."""
 
     def __init__(self, script, lanes, device="cuda", record=False, po_signals=None, grid=0,
-                 wo_slots=None, lanes_per_item=0):
+                 wo_slots=None, lanes_per_item=0, planned=True):
         self.script = script
         self.lanes = lanes
         self.device = torch.device(device)
         self.ds = sim.DeviceScript(script, self.device)
-        # the kernel reads the script in its own prepared layout, with the
-        # global-read sources resolved once
-        L = lib()
         n_parts = getattr(script, "num_partitions", None)
         if n_parts is None:
             n_parts = len(script.stage_block_part)
         self.num_partitions = int(n_parts)
-        self.prepared = torch.empty_like(self.ds.blocks_data)
-        self.part_base_dev = torch.empty(self.ds.num_blocks * self.ds.num_major_stages,
-                                         dtype=torch.int32, device=self.device)
-        self.gr_sources = torch.empty(L.jq_batched_gr_words(self.num_partitions), dtype=torch.int32,
-                                      device=self.device)
-        rc = L.jq_batched_prepare(self.ds.blocks_start.data_ptr(), self.ds.blocks_data.data_ptr(),
-                                  self.ds.blocks_data.numel(), self.ds.num_blocks,
-                                  self.ds.num_major_stages, self.num_partitions,
-                                  self.prepared.data_ptr(), self.part_base_dev.data_ptr(),
-                                  self.gr_sources.data_ptr(),
-                                  torch.cuda.current_stream(self.device).cuda_stream)
-        if rc:
-            raise RuntimeError("jq_batched_prepare: " + sim.lib().jq_strerror(rc).decode())
+        self._prep = None
         self.eff = getattr(script, "effective_words", None) or \
             script.reg_io_state_size * (2 if script.xprop_enabled else 1)
         self.sig = self.eff * 32
@@ -219,6 +223,19 @@ class BatchedSim:
                 raise ValueError(f"octet items need an X-propagating script, lanes divisible by 8 "
                                  f"and every partition within {cap} slots (needs {need:#x})")
             self.x_interleaved = 2
+        # the gate-list plan in the items asked for, or the widest that the
+        # lanes divide into; without one the prepared script runs
+        self.plan = self._plan_ws = None
+        if planned and wo_slots is None:
+            forms = [w for w in (8, 2, 1) if lanes % w == 0 and lanes_per_item in (0, w)]
+            for w in forms:
+                layout = (2 if script.xprop_enabled else 3) if w == 8 else \
+                    (1 if script.xprop_enabled else 0)
+                if self._build_plan(w, layout):
+                    self.x_interleaved = layout
+                    break
+        if self.plan is None:
+            self._prepared()
         regions = getattr(script, "input_regions", None)
         if regions is None:
             self.in_sigs = input_words(script) * 32
@@ -235,7 +252,7 @@ class BatchedSim:
         self.block_list_start = torch.from_numpy(bls.view(np.int32)).to(self.device)
         self.sram_words = max(1, script.sram_storage_size)
         n_streams = 32 * lanes
-        self.state_a = torch.zeros(L.jq_batched_state_words(lanes, self.sig), dtype=torch.int32,
+        self.state_a = torch.zeros(lib().jq_batched_state_words(lanes, self.sig), dtype=torch.int32,
                                    device=self.device)
         self.state_b = torch.zeros_like(self.state_a)
         self.sram = torch.zeros(n_streams * self.sram_words, dtype=torch.int32, device=self.device)
@@ -248,6 +265,60 @@ class BatchedSim:
         # lane words per work item: 0 lets the library pick (lane pairs when
         # lanes is even and they fit), 1, 2 or 8 (octets) forces one
         self.lanes_per_item = lanes_per_item
+
+    def _prepared(self):
+        """(prepared script, global-read sources, first partition of each
+        entry): the layout that the kernels for scripts without a plan read
+        (jq_batched_prepare), made on first use."""
+        if self._prep is None:
+            L = lib()
+            ds, dev = self.ds, self.device
+            prepared = torch.empty_like(ds.blocks_data)
+            part_base = torch.empty(ds.num_blocks * ds.num_major_stages, dtype=torch.int32, device=dev)
+            gr = torch.empty(L.jq_batched_gr_words(self.num_partitions), dtype=torch.int32, device=dev)
+            rc = L.jq_batched_prepare(ds.blocks_start.data_ptr(), ds.blocks_data.data_ptr(),
+                                      ds.blocks_data.numel(), ds.num_blocks, ds.num_major_stages,
+                                      self.num_partitions, prepared.data_ptr(), part_base.data_ptr(),
+                                      gr.data_ptr(), torch.cuda.current_stream(dev).cuda_stream)
+            if rc:
+                raise RuntimeError("jq_batched_prepare: " + sim.lib().jq_strerror(rc).decode())
+            self._prep = (prepared, gr, part_base)
+        return self._prep
+
+    prepared = property(lambda self: self._prepared()[0])
+    gr_sources = property(lambda self: self._prepared()[1])
+    part_base_dev = property(lambda self: self._prepared()[2])
+
+    def _build_plan(self, lanes_per_item, layout):
+        """True when the script has a plan for items of lanes_per_item lane
+        words in this state layout (jq_batched_plan_build)."""
+        L = lib()
+        rio = self.eff // (2 if self.script.xprop_enabled else 1)
+        if self.eff * 32 != self.sig or rio * (2 if self.script.xprop_enabled else 1) != self.eff:
+            return False
+        n = L.jq_batched_plan_words(self.ds.blocks_data.numel(), self.ds.num_blocks,
+                                    self.ds.num_major_stages, rio)
+        ws = torch.empty(n, dtype=torch.int32, device=self.device)
+        p = BatchedPlan()
+        rc = L.jq_batched_plan_build(self.ds.blocks_start.data_ptr(), self.ds.blocks_data.data_ptr(),
+                                     self.ds.num_blocks, self.ds.num_major_stages, rio, self.lanes,
+                                     lanes_per_item, layout, ws.data_ptr(), n, ctypes.byref(p),
+                                     torch.cuda.current_stream(self.device).cuda_stream)
+        if rc:
+            raise RuntimeError("jq_batched_plan_build: " + sim.lib().jq_strerror(rc).decode())
+        if not p.supported or p.num_partitions != self.num_partitions:
+            return False
+        used = ws[:p.used_words].clone()  # the used part only
+        for f in ("blob", "item_off", "item_words"):
+            setattr(p, f, getattr(p, f) - ws.data_ptr() + used.data_ptr())
+        torch.cuda.current_stream(self.device).synchronize()
+        self.plan, self._plan_ws = p, used
+        return True
+
+    def plan_words(self):
+        """Words of the plan's item blobs: what a cycle streams of the script."""
+        lo = (self.plan.item_words - self._plan_ws.data_ptr()) // 4
+        return int(self._plan_ws[lo:lo + self.plan.stage_item[32]].sum())
 
     def octet_need(self):
         """The most 64-byte tree slots an octet item needs for any partition
@@ -300,8 +371,10 @@ class BatchedSim:
         checks per stream into its event buffer), or None."""
         L = lib()
         wave_ptr = wave.data_ptr() if wave is not None else None
+        prepared, gr, base = (None, None, None) if self.plan is not None else \
+            (t.data_ptr() for t in self._prepared())
         a = BatchArgs(self.ds.num_blocks, self.ds.num_major_stages, self.ds.blocks_start.data_ptr(),
-                      self.prepared.data_ptr(), self.lanes, self.sram.data_ptr(),
+                      prepared, self.lanes, self.sram.data_ptr(),
                       self.sram_x.data_ptr(), self.sram_words, cycles, self.sig,
                       self.state_a.data_ptr(), self.state_b.data_ptr(),
                       stim.data_ptr() if stim is not None else None, self.in_sigs,
@@ -311,8 +384,7 @@ class BatchedSim:
                       record_buf.data_ptr() if record_buf is not None else None,
                       self.wo_slots, self.block_list.data_ptr(), self.block_list_start.data_ptr(),
                       part_cycles.data_ptr() if part_cycles is not None else None,
-                      self.part_base_dev.data_ptr(), self.gr_sources.data_ptr(),
-                      self.grid, barrier_timeout_cycles,
+                      base, gr, self.grid, barrier_timeout_cycles,
                       stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream,
                       self.lanes_per_item, self.x_interleaved)
         if timing is not None:
@@ -322,7 +394,8 @@ class BatchedSim:
             a.events = timing.events.data_ptr()
             a.event_capacity = timing.capacity
             a.first_cycle = first_cycle
-        rc = L.jq_simulate_batched(ctypes.byref(a))
+        rc = L.jq_simulate_batched_planned(ctypes.byref(a), ctypes.byref(self.plan)) \
+            if self.plan is not None else L.jq_simulate_batched(ctypes.byref(a))
         if rc:
             raise RuntimeError("jq_simulate_batched: " + sim.lib().jq_strerror(rc).decode())
 

@@ -32,6 +32,7 @@
 // each script block's execution order), so the caller computes the arrival
 // tables once with the plain interpreter, and only the clock-enable gate of
 // the check differs between streams.
+#include "plan_build.cuh"
 #include "sim_common.cuh"
 
 #include <cstdio>
@@ -180,9 +181,11 @@ __host__ __device__ __forceinline__ uint32_t owned_pos(uint32_t u, int i) {
 //   layout 2, lane octets (X interleaved): ((l >> 3) * V + s mod V) * 16 +
 //     2 * (l & 7) + (s >= V), i.e. the 64 bytes (v0, x0, ..., v7, x7) of a
 //     signal for 8 lane words (256 streams) are adjacent;
-//   layout 0, lane pairs without X: ((l >> 1) * sig + s) * 2 + (l & 1).
+//   layout 0, lane pairs without X: ((l >> 1) * sig + s) * 2 + (l & 1);
+//   layout 3, lane octets without X: ((l >> 3) * sig + s) * 8 + (l & 7).
 __host__ __device__ __forceinline__ size_t phys(int layout, size_t vsig, size_t sig, uint32_t l,
                                                 size_t s) {
+  if (layout == 3) return ((((size_t)(l >> 3)) * sig + s) << 3) + (l & 7);
   if (layout) {
     const bool x = s >= vsig;
     const size_t sv = x ? s - vsig : s;
@@ -2348,6 +2351,8 @@ __global__ void jq_batched_count_kernel(const size_t *blocks_start, const uint32
 
 }  // namespace jqk
 
+#include "batched_plan.cuh"
+
 using namespace jqk;
 
 // Lane-major [lane][signal] snapshot <-> the interleaved batched state.
@@ -2470,8 +2475,9 @@ size_t jq_batched_state_words(uint32_t lanes, size_t signals) {
 
 static int pack_launch(const uint32_t *src, uint32_t *dst, uint32_t lanes, size_t signals,
                        int32_t x_interleaved, int unpack, void *stream) {
-  if (!src || !dst || lanes == 0 || signals == 0 || x_interleaved < 0 || x_interleaved > 2 ||
-      (x_interleaved && (signals & 1)) || (x_interleaved == 2 && lanes % 8))
+  if (!src || !dst || lanes == 0 || signals == 0 || x_interleaved < 0 || x_interleaved > 3 ||
+      ((x_interleaved == 1 || x_interleaved == 2) && (signals & 1)) ||
+      (x_interleaved >= 2 && lanes % 8))
     return JQ_ERR_INVALID_ARG;
   const size_t n = (size_t)lanes * signals;
   const unsigned grid = (unsigned)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
@@ -2554,6 +2560,51 @@ int jq_batched_slot_need(const size_t *blocks_start, const uint32_t *prepared, s
   return cudaGetLastError() == cudaSuccess ? JQ_OK : JQ_ERR_LAUNCH;
 }
 
+// Kernel parameters of a launch, all but its barrier slot.
+static int fill_params(const jq_batch_args *a, uint32_t wo_slots, BatchParams &P) {
+  P.num_blocks = (unsigned)a->num_blocks;
+  P.num_major_stages = (unsigned)a->num_major_stages;
+  P.lanes = a->lanes;
+  P.blocks_start = a->blocks_start;
+  P.blocks_data = a->blocks_data;
+  P.sram = a->sram_data;
+  P.sram_x = a->sram_xmask;
+  P.sram_words = a->sram_words_per_stream;
+  P.num_cycles = a->num_cycles;
+  P.sig_per_snap = a->signals_per_snapshot;
+  if ((a->x_interleaved == 1 || a->x_interleaved == 2) && (P.sig_per_snap & 1)) return JQ_ERR_INVALID_ARG;
+  P.xhalf = a->x_interleaved == 1 || a->x_interleaved == 2;
+  P.layout = a->x_interleaved;
+  P.slot_cap = 0;
+  P.vsig = P.xhalf ? P.sig_per_snap / 2 : P.sig_per_snap;
+  P.state_a = a->state_a;
+  P.state_b = a->state_b;
+  P.stim = a->stimulus;
+  P.input_sigs = a->input_signals;
+  P.input_regions = a->input_regions;
+  P.n_input_regions = a->n_input_regions;
+  P.po_sig = a->po_signals;
+  P.n_po = a->n_po;
+  P.wave = a->wave;
+  P.record = a->record;
+  P.wo_slots = wo_slots;
+  P.block_list = a->block_list;
+  P.block_list_start = a->block_list_start;
+  P.part_cycles = a->part_cycles;
+  P.part_base = a->part_base;
+  P.gr_sources = a->gr_sources;
+  P.constraints = a->timing_constraints;
+  P.arr_first = a->arrival_first;
+  P.arr_steady = a->arrival_steady;
+  P.events = a->events;
+  P.event_cap = a->event_capacity;
+  P.first_cycle = a->first_cycle;
+  if (P.constraints && (!P.arr_first || !P.arr_steady || !P.events)) return JQ_ERR_INVALID_ARG;
+  P.timeout = a->barrier_timeout_cycles ? a->barrier_timeout_cycles : DEFAULT_BARRIER_TIMEOUT;
+  P.chunk_timeout = DEFAULT_BARRIER_TIMEOUT;
+  return JQ_OK;
+}
+
 int jq_simulate_batched(const jq_batch_args *a) {
   if (!a || a->lanes == 0 || a->num_blocks == 0 || a->num_major_stages == 0 ||
       a->num_major_stages > 32 || !a->state_a || !a->state_b || a->wo_slots > 256 ||
@@ -2573,47 +2624,10 @@ int jq_simulate_batched(const jq_batch_args *a) {
   size_t grid = a->grid ? a->grid : maxg;
   if (grid > maxg) return JQ_ERR_TOO_MANY_BLOCKS;
   BatchParams P;
-  P.num_blocks = (unsigned)a->num_blocks;
-  P.num_major_stages = (unsigned)a->num_major_stages;
-  P.lanes = a->lanes;
-  P.blocks_start = a->blocks_start;
-  P.blocks_data = a->blocks_data;
-  P.sram = a->sram_data;
-  P.sram_x = a->sram_xmask;
-  P.sram_words = a->sram_words_per_stream;
-  P.num_cycles = a->num_cycles;
-  P.sig_per_snap = a->signals_per_snapshot;
-  if (a->x_interleaved && (P.sig_per_snap & 1)) return JQ_ERR_INVALID_ARG;
-  P.xhalf = a->x_interleaved != 0;
-  P.layout = a->x_interleaved;
+  const int rc = fill_params(a, wo_slots, P);
+  if (rc != JQ_OK) return rc;
   P.slot_cap = v.nl == 8 ? oct_slot_capacity() : 0;
-  P.vsig = P.xhalf ? P.sig_per_snap / 2 : P.sig_per_snap;
-  P.state_a = a->state_a;
-  P.state_b = a->state_b;
-  P.stim = a->stimulus;
-  P.input_sigs = a->input_signals;
-  P.input_regions = a->input_regions;
-  P.n_input_regions = a->n_input_regions;
-  P.po_sig = a->po_signals;
-  P.n_po = a->n_po;
-  P.wave = a->wave;
-  P.record = a->record;
-  P.wo_slots = wo_slots;
-  P.block_list = a->block_list;
-  P.block_list_start = a->block_list_start;
-  P.part_cycles = a->part_cycles;
-  P.part_base = a->part_base;
-  P.gr_sources = a->gr_sources;
   if (!P.part_base || !P.gr_sources) return JQ_ERR_INVALID_ARG;
-  P.constraints = a->timing_constraints;
-  P.arr_first = a->arrival_first;
-  P.arr_steady = a->arrival_steady;
-  P.events = a->events;
-  P.event_cap = a->event_capacity;
-  P.first_cycle = a->first_cycle;
-  if (P.constraints && (!P.arr_first || !P.arr_steady || !P.events)) return JQ_ERR_INVALID_ARG;
-  P.timeout = a->barrier_timeout_cycles ? a->barrier_timeout_cycles : DEFAULT_BARRIER_TIMEOUT;
-  P.chunk_timeout = DEFAULT_BARRIER_TIMEOUT;
   P.slot = launch_slot(a->stream, true);
   if (P.slot < 0) return JQ_ERR_TOO_MANY_STREAMS;
   jq_batched_reset_kernel<<<1, 1, 0, st>>>(P.slot);
@@ -2622,6 +2636,116 @@ int jq_simulate_batched(const jq_batch_args *a) {
   void *args[] = {&P};
   cudaError_t e = cudaLaunchCooperativeKernel(variant_fn(v), (unsigned)grid, BT, args, smem, st);
   return e == cudaSuccess ? JQ_OK : JQ_ERR_LAUNCH;
+}
+
+// ---- gate-list plan (batched_plan.cuh)
+
+static const void *bplan_fn(uint32_t lw, bool x) {
+  if (lw == 8)
+    return x ? (const void *)jq_bplan_kernel<8, true> : (const void *)jq_bplan_kernel<8, false>;
+  if (lw == 2)
+    return x ? (const void *)jq_bplan_kernel<2, true> : (const void *)jq_bplan_kernel<2, false>;
+  return x ? (const void *)jq_bplan_kernel<1, true> : (const void *)jq_bplan_kernel<1, false>;
+}
+
+static size_t bplan_smem(const jq_batched_plan *p, uint32_t nbuf) {
+  const size_t wps = p->lanes_per_item * (p->with_x ? 2 : 1);
+  return 4 * (size_t)nbuf * p->max_blob + 4 * wps * p->max_slots + 4 * 256 * (size_t)p->lanes_per_item;
+}
+
+size_t jq_batched_plan_words(size_t blocks_data_len, size_t num_blocks, size_t num_major_stages,
+                             size_t state_words) {
+  return plan_workspace_words(blocks_data_len, num_blocks, num_major_stages, state_words);
+}
+
+int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_data,
+                          size_t num_blocks, size_t num_major_stages, size_t state_words,
+                          uint32_t lanes, uint32_t lanes_per_item, int32_t x_interleaved,
+                          uint32_t *workspace, size_t workspace_words, jq_batched_plan *plan,
+                          void *stream) {
+  const bool x = x_interleaved == 1 || x_interleaved == 2;
+  if (!blocks_start || !blocks_data || !workspace || !plan || num_blocks == 0 ||
+      num_major_stages == 0 || num_major_stages > 32 || state_words >= PLAN_DIRECT / 32 ||
+      lanes == 0 || x_interleaved < 0 || x_interleaved > 3 ||
+      (lanes_per_item != 1 && lanes_per_item != 2 && lanes_per_item != 8) ||
+      lanes % lanes_per_item || (lanes_per_item == 8) != (x_interleaved >= 2))
+    return JQ_ERR_INVALID_ARG;
+  *plan = jq_batched_plan{};
+  plan->num_major_stages = num_major_stages;
+  plan->lanes = lanes;
+  plan->lanes_per_item = lanes_per_item;
+  plan->x_interleaved = x_interleaved;
+  plan->with_x = x;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return JQ_ERR_LAUNCH;
+  PlanBuilder b{blocks_start, blocks_data, num_blocks, num_major_stages, state_words,
+                workspace, workspace_words, (cudaStream_t)stream};
+  bool ok = false;
+  int rc = b.scan(&ok);
+  if (rc != JQ_OK || !ok) return rc;
+  plan->num_partitions = b.parts;
+  if ((b.r.x_use & 2u) && (!x || b.r.xoff_max != state_words)) return JQ_OK;
+  const size_t groups = lanes / lanes_per_item;
+  const size_t round = (size_t)sms > groups ? (size_t)sms / groups : 1;
+  const size_t lim = plan_smem_limit(bplan_fn(lanes_per_item, x));
+  // one item per CTA where a stage has few partitions, more parts where an
+  // item's slots do not fit
+  for (size_t want = round;; want *= 2) {
+    rc = b.build(PLAN_SIGNALS, want, round, &ok);
+    if (rc != JQ_OK) return rc;
+    if (ok) {
+      plan->max_blob = b.r.max_blob;
+      plan->max_slots = b.r.max_slots;
+      plan->nbuf = bplan_smem(plan, 2) <= lim ? 2 : bplan_smem(plan, 1) <= lim ? 1 : 0;
+      plan->widest = b.widest;
+      for (size_t ms = 0; ms <= 32; ++ms) plan->stage_item[ms] = b.stage_item[ms];
+      plan->used_words = b.used_words;
+      plan->blob = b.blob;
+      plan->item_off = b.item_off;
+      plan->item_words = b.item_words;
+      plan->supported = plan->nbuf != 0;
+    }
+    if (plan->supported || want >= PLAN_MAX_NSUB * b.most) return JQ_OK;
+  }
+}
+
+int jq_simulate_batched_planned(const jq_batch_args *a, const jq_batched_plan *p) {
+  if (!a || !p || !p->supported || a->lanes != p->lanes || a->x_interleaved != p->x_interleaved ||
+      a->num_major_stages != p->num_major_stages || !a->state_a || !a->state_b ||
+      a->input_signals >> 31 || (a->n_po && (!a->po_signals || !a->wave)))
+    return JQ_ERR_INVALID_ARG;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return JQ_ERR_LAUNCH;
+  const size_t grid = a->grid ? a->grid : (size_t)sms;
+  if (grid > (size_t)sms) return JQ_ERR_TOO_MANY_BLOCKS;
+  BatchParams P;
+  int rc = fill_params(a, 0, P);
+  if (rc != JQ_OK) return rc;
+  BPlanParams Q;
+  Q.blob = p->blob;
+  Q.item_off = p->item_off;
+  Q.item_words = p->item_words;
+  for (size_t ms = 0; ms <= 32; ++ms) Q.stage_item[ms] = p->stage_item[ms];
+  Q.blob_cap = p->max_blob;
+  Q.nbuf = p->nbuf;
+  Q.slots = p->max_slots;
+  P.slot = launch_slot(a->stream, true);
+  if (P.slot < 0) return JQ_ERR_TOO_MANY_STREAMS;
+  cudaStream_t st = (cudaStream_t)a->stream;
+  const void *fn = bplan_fn(p->lanes_per_item, p->with_x);
+  const int smem = (int)bplan_smem(p, p->nbuf);
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    return JQ_ERR_LAUNCH;
+  jq_batched_reset_kernel<<<1, 1, 0, st>>>(P.slot);
+  if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
+  void *args[] = {&P, &Q};
+  return cudaLaunchCooperativeKernel(fn, (unsigned)grid, BT, args, smem, st) == cudaSuccess
+             ? JQ_OK
+             : JQ_ERR_LAUNCH;
 }
 
 int jq_batched_status(void *stream) {

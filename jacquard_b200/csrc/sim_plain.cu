@@ -424,7 +424,6 @@ __global__ void __launch_bounds__(NT) jq_plain_depth_kernel(const size_t *blocks
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
-#include <vector>
 
 using namespace jqk;
 
@@ -494,29 +493,6 @@ int plain_prepare(const size_t *blocks_start, const uint32_t *blocks_data, size_
   return rc;
 }
 
-// Layout of the plan build's workspace (words; the blobs take the rest).
-struct PlanLayout {
-  size_t part_base, part_ms, part_off, writer, unwritten, items, item_words, item_off, blob;
-  PlanLayout(size_t entries, size_t parts, size_t n_items, size_t writer_words) {
-    size_t w = (sizeof(PlanResult) / 4 + 3) & ~(size_t)3;
-    auto take = [&](size_t n) {
-      const size_t at = w;
-      w += (n + 3) & ~(size_t)3;
-      return at;
-    };
-    part_base = take(entries);
-    part_ms = take(parts);
-    part_off = take(2 * parts);
-    writer = take(writer_words);
-    unwritten = take(writer_words);
-    items = take(2 * n_items);
-    item_words = take(n_items);
-    item_off = take(2 * n_items);
-    blob = w;
-  }
-};
-constexpr size_t PLAN_MIN_PART = 256 + 3 * (size_t)STAGE_WORDS;  // words of the smallest partition
-constexpr size_t PLAN_MAX_NSUB = 16;
 // Items a stage's partitions are split towards: one per SM (2M-gate SoC, 32
 // partitions a stage: 5.8 us a stage unsplit, 4.9 at 64 items, 4.8 at 128;
 // 256k-gate SoC, 3 partitions: 5.0 unsplit, 2.5 at 48).
@@ -546,17 +522,6 @@ const void *plan_fn(const jq_plain_plan *p) {
     return p->xoff ? (const void *)plan_mirror_kernel<true>
                    : (const void *)plan_mirror_kernel<false>;
   return p->xoff ? (const void *)plan_flow_kernel<true> : (const void *)plan_flow_kernel<false>;
-}
-
-// Opt-in shared memory per CTA left for the dynamic part of fn.
-size_t plan_smem_limit(const void *fn) {
-  int dev = 0, optin = 0;
-  cudaFuncAttributes fa;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
-      cudaFuncGetAttributes(&fa, fn) != cudaSuccess || (size_t)optin < fa.sharedSizeBytes)
-    return 0;
-  return (size_t)optin - fa.sharedSizeBytes;
 }
 
 // Launch of the mirrored form: one cluster of the next power of two CTAs.
@@ -597,129 +562,40 @@ int plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t n
   *plan = jq_plain_plan{};
   plan->num_blocks = num_blocks;
   plan->num_major_stages = nms;
-  const size_t entries = num_blocks * nms;
-  const PlanLayout l0(entries, 0, 0, 0);
-  if (ws_words < l0.blob) return JQ_ERR_INVALID_ARG;
-  std::vector<uint32_t> h(entries), base(entries);
-  plan_count_kernel<<<(unsigned)((entries + 255) / 256), 256, 0, st>>>(
-      blocks_start, blocks_data, ws + l0.part_base, (unsigned)entries);
-  if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
-  if (cudaMemcpyAsync(h.data(), ws + l0.part_base, entries * 4, cudaMemcpyDeviceToHost, st) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return JQ_ERR_CUDA;
-  size_t parts = 0, most = 0;
-  std::vector<size_t> per_stage(nms, 0);
-  for (size_t ms = 0; ms < nms; ++ms) {
-    for (size_t b = 0; b < num_blocks; ++b) {
-      base[ms * num_blocks + b] = (uint32_t)(parts + per_stage[ms]);
-      per_stage[ms] += h[ms * num_blocks + b] & 0x7fffffffu;
-    }
-    parts += per_stage[ms];
-    most = per_stage[ms] > most ? per_stage[ms] : most;
-  }
-  if (parts == 0) return JQ_OK;  // nothing to run: not supported
-  const PlanLayout l1(entries, parts, 0, state_words);
-  if (ws_words < l1.blob) return JQ_OK;
-  PlanResult *res = reinterpret_cast<PlanResult *>(ws), r;
-  unsigned long long *part_off = reinterpret_cast<unsigned long long *>(ws + l1.part_off);
-  if (cudaMemsetAsync(res, 0, sizeof(PlanResult), st) != cudaSuccess ||
-      cudaMemsetAsync(ws + l1.writer, 0, state_words * 4, st) != cudaSuccess ||
-      cudaMemcpyAsync(ws + l1.part_base, base.data(), entries * 4, cudaMemcpyHostToDevice, st) !=
-          cudaSuccess)
-    return JQ_ERR_CUDA;
-  plan_list_kernel<<<(unsigned)entries, 64, 0, st>>>(
-      blocks_start, blocks_data, ws + l1.part_base, (unsigned)entries, (unsigned)num_blocks,
-      part_off, ws + l1.part_ms, ws + l1.writer, (uint32_t)state_words, res);
-  plan_unwritten_kernel<<<64, 256, 0, st>>>(ws + l1.writer, (uint32_t)state_words,
-                                            ws + l1.unwritten, (uint32_t)state_words, res);
-  if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
-  if (cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return JQ_ERR_CUDA;
-  if (r.unsupported) return JQ_OK;
-  plan->rio = r.rio;
-  plan->xoff = (r.x_use & 2u) ? r.xoff_max : 0;
-  plan->n_unwritten = r.n_unwritten;
-  plan->unwritten = ws + l1.unwritten;
-  for (size_t ms = 0; ms < nms; ++ms) plan->stage_words[ms] = r.stage_words[ms];
-  const bool one_xoff = !(r.x_use & 2u) || (r.xoff_max == ~r.xoff_inv_max && r.xoff_max > 0);
-  if (!one_xoff) return JQ_OK;
-  bool mirrored = most <= PLAN_MIRROR_PARTS && target != PLAN_GRID_ONLY &&
-                  2 * (size_t)r.rio * (plan->xoff ? 8 : 4) <= PLAN_MIRROR_BYTES;
-  const int smem = (int)sizeof(PlanShared);
-  if (cudaFuncSetAttribute(plan_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-      cudaSuccess)
-    return JQ_ERR_LAUNCH;
+  PlanBuilder b{blocks_start, blocks_data, num_blocks, nms, state_words, ws, ws_words, st};
+  bool ok = false;
+  int rc = b.scan(&ok);
+  if (rc != JQ_OK || !ok) return rc;
+  plan->rio = b.r.rio;
+  plan->xoff = (b.r.x_use & 2u) ? b.r.xoff_max : 0;
+  plan->n_unwritten = b.r.n_unwritten;
+  plan->unwritten = b.unwritten();
+  for (size_t ms = 0; ms < nms; ++ms) plan->stage_words[ms] = b.r.stage_words[ms];
+  bool mirrored = b.most <= PLAN_MIRROR_PARTS && target != PLAN_GRID_ONLY &&
+                  2 * (size_t)b.r.rio * (plan->xoff ? 8 : 4) <= PLAN_MIRROR_BYTES;
   for (;; mirrored = false) {
-    // items: partitions, split where a stage has few of them
     const size_t want = target && target != PLAN_GRID_ONLY ? target
                         : mirrored                         ? PLAN_CLUSTER
                                                            : PLAN_GRID_ITEMS;
-    std::vector<uint32_t> items;
-    plan->widest = 1;
-    size_t pid = 0;
-    for (size_t ms = 0; ms < nms; ++ms) {
-      size_t nsub = per_stage[ms] ? want / per_stage[ms] : 1;
-      nsub = nsub < 1 ? 1 : nsub > PLAN_MAX_NSUB ? PLAN_MAX_NSUB : nsub;
-      plan->stage_item[ms] = (uint32_t)(items.size() / 2);
-      for (size_t b = 0; b < num_blocks; ++b) {
-        const uint32_t c = h[ms * num_blocks + b];
-        // an entry with an SRAM partition is not split
-        const uint32_t ks = (c >> 31) ? 1u : (uint32_t)nsub;
-        for (uint32_t k = 0; k < (c & 0x7fffffffu); ++k, ++pid)
-          for (uint32_t s = 0; s < ks; ++s) {
-            items.push_back((uint32_t)pid);
-            items.push_back(s | ks << 16);
-          }
-      }
-      const uint32_t n = (uint32_t)(items.size() / 2) - plan->stage_item[ms];
-      plan->widest = n > plan->widest ? n : plan->widest;
-    }
-    const size_t n_items = items.size() / 2;
-    for (size_t ms = nms; ms <= 32; ++ms) plan->stage_item[ms] = (uint32_t)n_items;
-    const PlanLayout lay(entries, parts, n_items, state_words);
-    if (ws_words < lay.blob + 4) return JQ_OK;
-    r.unsupported = 0;
-    r.used = 0;
-    r.max_blob = r.max_slots = r.max_gw = 0;
-    if (cudaMemcpyAsync(res, &r, sizeof r, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(ws + lay.items, items.data(), items.size() * 4, cudaMemcpyHostToDevice,
-                        st) != cudaSuccess)
-      return JQ_ERR_CUDA;
-    PlanBuildParams B;
-    B.script = blocks_data;
-    B.part_off = part_off;
-    B.part_ms = ws + lay.part_ms;
-    B.items = ws + lay.items;
-    B.writer = ws + lay.writer;
-    B.writer_words = (uint32_t)state_words;
-    B.direct = mirrored;
-    B.blob = ws + lay.blob;
-    B.blob_cap = ws_words - lay.blob;
-    B.item_off = reinterpret_cast<unsigned long long *>(ws + lay.item_off);
-    B.item_words = ws + lay.item_words;
-    B.res = res;
-    plan_build_kernel<<<(unsigned)n_items, PB, smem, st>>>(B, (uint32_t)n_items);
-    if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
-    if (cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return JQ_ERR_CUDA;
-    plan->mirrored = mirrored;
-    plan->exchange_words = mirrored ? 0 : 4 * (size_t)r.rio * (plan->xoff ? 4 : 2);
-    plan->max_blob = r.max_blob;
-    plan->max_slots = r.max_slots;
-    plan->max_gw = r.max_gw;
-    plan->used_words = lay.blob + (size_t)r.used;
-    plan->blob = ws + lay.blob;
-    plan->item_off = B.item_off;
-    plan->item_words = B.item_words;
-    if (!(r.unsupported & 1u)) {
+    rc = b.build(mirrored ? PLAN_MIRROR : PLAN_WORDS, want, 0, &ok);
+    if (rc != JQ_OK) return rc;
+    if (ok) {
+      plan->mirrored = mirrored;
+      plan->exchange_words = mirrored ? 0 : 4 * (size_t)b.r.rio * (plan->xoff ? 4 : 2);
+      plan->max_blob = b.r.max_blob;
+      plan->max_slots = b.r.max_slots;
+      plan->max_gw = b.r.max_gw;
+      for (size_t ms = 0; ms <= 32; ++ms) plan->stage_item[ms] = b.stage_item[ms];
+      plan->widest = b.widest;
+      plan->used_words = b.used_words;
+      plan->blob = b.blob;
+      plan->item_off = b.item_off;
+      plan->item_words = b.item_words;
       const size_t lim = plan_smem_limit(plan_fn(plan));
       plan->nbuf = plan_smem_bytes(plan, 2) <= lim ? 2 : plan_smem_bytes(plan, 1) <= lim ? 1 : 0;
-      plan->supported = plan->nbuf && !r.unsupported &&
-                        (!mirrored || (plan->widest <= PLAN_CLUSTER &&
-                                       plan_cluster_launch(plan, nullptr, st, true) == JQ_OK));
+      plan->supported = plan->nbuf && (!mirrored || (plan->widest <= PLAN_CLUSTER &&
+                                                     plan_cluster_launch(plan, nullptr, st, true) ==
+                                                         JQ_OK));
     }
     if (plan->supported || !mirrored) return JQ_OK;
   }
@@ -1004,10 +880,7 @@ int jq_plain_prepare(const size_t *blocks_start, const uint32_t *blocks_data, si
 
 size_t jq_plain_plan_words(size_t blocks_data_len, size_t num_blocks, size_t num_major_stages,
                            size_t state_words) {
-  const size_t entries = num_blocks * num_major_stages;
-  const size_t parts = blocks_data_len / PLAN_MIN_PART + 1;
-  return PlanLayout(entries, parts, parts + num_major_stages * PLAN_GRID_ITEMS, state_words).blob +
-         blocks_data_len / 2 + 4096;
+  return plan_workspace_words(blocks_data_len, num_blocks, num_major_stages, state_words);
 }
 
 int jq_plain_plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t num_blocks,
