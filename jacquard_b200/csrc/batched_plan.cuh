@@ -152,13 +152,47 @@ __device__ __forceinline__ uint32_t bp_word(uint4 v, int i) {
 __device__ __forceinline__ uint32_t bp_word(uint2 v, int i) { return i ? v.y : v.x; }
 __device__ __forceinline__ uint32_t bp_word(uint32_t v, int) { return v; }
 
-// Setup/hold checks of one state word for all lane words of an item (cold).
-__device__ __noinline__ void bp_check(const BatchParams &P, uint32_t word, const uint32_t *clk,
-                                      uint32_t lw, uint32_t lane0, uint32_t cyc) {
+// Setup/hold checks of one state word for the lane words of an item, with the
+// plain interpreter's predicate (csrc/kernel_v1_impl.cuh:536-558) per stream:
+// arrival a and constraint cv are the word's, clk[l] the streams of lane word
+// l whose clock enable is set on any of its signals.  One warp; one atomic
+// claims the records of a kind.
+__device__ __noinline__ void bp_check(const BatchParams &P, uint32_t word, uint32_t a, uint32_t cv,
+                                      const uint32_t *clk, uint32_t lw, uint32_t lane0,
+                                      uint32_t cyc) {
+  const uint32_t clock_ps = __ldg(P.constraints), su = cv >> 16, ho = cv & 0xffffu;
+  const bool v[2] = {a > 0 && a + su > clock_ps, a < ho};
+  if (!cv || !(v[0] || v[1])) return;
+  const uint32_t lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+  // records as two 16-byte stores where the buffer's alignment allows it
+  const bool wide = (reinterpret_cast<size_t>(P.events->events) & 15) == 0;
+  uint32_t n = 0;
+  for (uint32_t l = 0; l < lw; ++l) n += __popc(clk[l]);
+  if (!n) return;
 #pragma unroll 1
-  for (uint32_t l = 0; l < lw; l += 2)
-    check_word(P, word, clk[l], lane0 + l, l + 1 < lw ? clk[l + 1] : 0u, lane0 + l + 1,
-               P.first_cycle + cyc, cyc == 0);
+  for (int kind = 0; kind < 2; ++kind) {
+    if (!v[kind]) continue;
+    const uint32_t slack = kind == 0 ? (uint32_t)((int32_t)clock_ps - (int32_t)a - (int32_t)su)
+                                     : (uint32_t)((int32_t)a - (int32_t)ho);
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&P.events->count, n);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll 1
+    for (uint32_t l = 0; l < lw; ++l) {
+      const uint32_t m = clk[l], idx = base + __popc(m & below);
+      if ((m >> lane) & 1u) {
+        if (wide && idx < P.event_cap) {
+          uint4 *e = reinterpret_cast<uint4 *>(&P.events->events[idx]);
+          e[0] = make_uint4(4 + kind, word, P.first_cycle + cyc, 32 * (lane0 + l) + lane);
+          e[1] = make_uint4(word, slack, a, kind == 0 ? su : ho);
+        } else {
+          put_event(P, idx, 4 + kind, word, P.first_cycle + cyc, slack, a, kind == 0 ? su : ho,
+                    32 * (lane0 + l) + lane);
+        }
+      }
+      base += __popc(m);
+    }
+  }
 }
 
 // Outputs and the optional record of the cycle that ended (state `in`), and
@@ -196,7 +230,7 @@ __device__ __noinline__ void bp_io(const BatchParams &P, const uint32_t *in, uin
   }
 }
 
-template <int LW, bool X>
+template <int LW, bool X, bool TIMED>
 __global__ void __launch_bounds__(BT, 1)
     jq_bplan_kernel(const __grid_constant__ BatchParams P, const __grid_constant__ BPlanParams Q) {
   using V = typename LaneVec<LW, X>::T;
@@ -213,7 +247,9 @@ __global__ void __launch_bounds__(BT, 1)
   uint32_t *const buf0 = reinterpret_cast<uint32_t *>(dyn);
   V *const S = reinterpret_cast<V *>(dyn + 4 * (size_t)Q.nbuf * Q.blob_cap);
   uint32_t *const Sw = reinterpret_cast<uint32_t *>(S);
-  uint32_t *const clk_or = Sw + (size_t)Q.slots * WPS;  // setup/hold checks: [256][LW]
+  // setup/hold checks: clock enables [256][LW], then (arrival, constraint) [256]
+  uint32_t *const clk_or = Sw + (size_t)Q.slots * WPS;
+  uint2 *const chk = reinterpret_cast<uint2 *>(clk_or + 256 * LW);
   const uint32_t t = threadIdx.x, k = t % TPE, el = t / TPE, warp = t >> 5, ln = t & 31;
   const uint32_t groups = P.lanes / LW, rank = blockIdx.x, G = gridDim.x, nms = P.num_major_stages;
   const bool two = Q.nbuf == 2;
@@ -313,7 +349,7 @@ __global__ void __launch_bounds__(BT, 1)
           break;
         }
         const long long t_start = clock64();
-        const uint32_t group = idx % groups, ngr = B[PH_NGR], nw = B[PH_NW];
+        const uint32_t group = groups == 1 ? 0 : idx % groups, ngr = B[PH_NGR], nw = B[PH_NW];
         const bool isx = X && B[PH_ISX] != 0;
         // the group's part of signal 0, in V units
         const size_t g0 = LW == 8   ? (size_t)group * P.vsig * TPE + k
@@ -352,8 +388,14 @@ __global__ void __launch_bounds__(BT, 1)
               }
             }
           }
-          if (P.constraints)
+          if constexpr (TIMED) {
             for (uint32_t i = t; i < nw * LW; i += BT) clk_or[i] = 0;
+            if (t < nw) {
+              const uint32_t o = B[PH_IO] + t;
+              chk[t] = make_uint2(__ldg((c ? P.arr_steady : P.arr_first) + o) & 0xffffu,
+                                  __ldg(P.constraints + 1 + o));
+            }
+          }
         }
         if (two && t == PT) issue();  // into the other buffer, free since the barrier above
         if (io) bp_io(P, in, out, c, g_rank, g_ctas, lane_lo, lane_n);
@@ -437,13 +479,13 @@ __global__ void __launch_bounds__(BT, 1)
               V old = v;
               if (bp_all<X>(en) != 0xffffffffu) old = __ldcg(vin + at);
               v = bp_commit<X>(v, old, en);
-              if (P.constraints) {
+              if constexpr (TIMED) {
 #pragma unroll
                 for (int j = 0; j < (int)(sizeof(V) / 4 / PV); ++j)
                   atomicOr(&clk_or[(q >> 5) * LW + k * (sizeof(V) / 4 / PV) + j],
                            bp_word(en, j * PV));
               }
-            } else if (P.constraints) {
+            } else if constexpr (TIMED) {
 #pragma unroll
               for (int j = 0; j < (int)(sizeof(V) / 4 / PV); ++j)
                 clk_or[(q >> 5) * LW + k * (sizeof(V) / 4 / PV) + j] = 0xffffffffu;
@@ -453,10 +495,11 @@ __global__ void __launch_bounds__(BT, 1)
             else
               vout[at] = v;
           }
-          if (P.constraints) {
+          if constexpr (TIMED) {
             __syncthreads();
             for (uint32_t j = warp; j < nw; j += BT / 32)
-              bp_check(P, B[PH_IO] + j, clk_or + j * LW, LW, group * LW, (uint32_t)c);
+              bp_check(P, B[PH_IO] + j, chk[j].x, chk[j].y, clk_or + j * LW, LW, group * LW,
+                       (uint32_t)c);
           }
         }
         if (P.part_cycles) {

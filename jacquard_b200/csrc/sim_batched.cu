@@ -2640,17 +2640,22 @@ int jq_simulate_batched(const jq_batch_args *a) {
 
 // ---- gate-list plan (batched_plan.cuh)
 
-static const void *bplan_fn(uint32_t lw, bool x) {
-  if (lw == 8)
-    return x ? (const void *)jq_bplan_kernel<8, true> : (const void *)jq_bplan_kernel<8, false>;
-  if (lw == 2)
-    return x ? (const void *)jq_bplan_kernel<2, true> : (const void *)jq_bplan_kernel<2, false>;
-  return x ? (const void *)jq_bplan_kernel<1, true> : (const void *)jq_bplan_kernel<1, false>;
+extern "C++" {
+template <bool X, bool TIMED>
+static const void *bplan_fn_of(uint32_t lw) {
+  return lw == 8   ? (const void *)jq_bplan_kernel<8, X, TIMED>
+         : lw == 2 ? (const void *)jq_bplan_kernel<2, X, TIMED>
+                   : (const void *)jq_bplan_kernel<1, X, TIMED>;
+}
+}
+static const void *bplan_fn(uint32_t lw, bool x, bool timed) {
+  if (timed) return x ? bplan_fn_of<true, true>(lw) : bplan_fn_of<false, true>(lw);
+  return x ? bplan_fn_of<true, false>(lw) : bplan_fn_of<false, false>(lw);
 }
 
 static size_t bplan_smem(const jq_batched_plan *p, uint32_t nbuf) {
   const size_t wps = p->lanes_per_item * (p->with_x ? 2 : 1);
-  return 4 * (size_t)nbuf * p->max_blob + 4 * wps * p->max_slots + 4 * 256 * (size_t)p->lanes_per_item;
+  return 4 * (size_t)nbuf * p->max_blob + 4 * wps * p->max_slots + 4 * 256 * (size_t)(p->lanes_per_item + 2);
 }
 
 size_t jq_batched_plan_words(size_t blocks_data_len, size_t num_blocks, size_t num_major_stages,
@@ -2689,7 +2694,7 @@ int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_dat
   if ((b.r.x_use & 2u) && (!x || b.r.xoff_max != state_words)) return JQ_OK;
   const size_t groups = lanes / lanes_per_item;
   const size_t round = (size_t)sms > groups ? (size_t)sms / groups : 1;
-  const size_t lim = plan_smem_limit(bplan_fn(lanes_per_item, x));
+  const size_t lim = plan_smem_limit(bplan_fn(lanes_per_item, x, true));
   // one item per CTA where a stage has few partitions, more parts where an
   // item's slots do not fit
   for (size_t want = round;; want *= 2) {
@@ -2736,7 +2741,7 @@ int jq_simulate_batched_planned(const jq_batch_args *a, const jq_batched_plan *p
   P.slot = launch_slot(a->stream, true);
   if (P.slot < 0) return JQ_ERR_TOO_MANY_STREAMS;
   cudaStream_t st = (cudaStream_t)a->stream;
-  const void *fn = bplan_fn(p->lanes_per_item, p->with_x);
+  const void *fn = bplan_fn(p->lanes_per_item, p->with_x, P.constraints != nullptr);
   const int smem = (int)bplan_smem(p, p->nbuf);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return JQ_ERR_LAUNCH;
