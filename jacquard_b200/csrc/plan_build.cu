@@ -29,6 +29,7 @@ struct PlanShared {
   uint32_t ref_a[8192], ref_b[8192];
   uint16_t woref[8192];
   uint32_t need[256], wneed[256], ext[256];
+  uint32_t top[PLAN_MAX_NS];  // lowest position of a stage read from outside, below 4096
   uint32_t lev[PLAN_MAX_LEVELS], lev_base[PLAN_MAX_LEVELS];
   uint32_t warp_sum[32];
   int bad;
@@ -170,17 +171,24 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   for (int ci = (int)ns - 1; ci >= 0; --ci) {
     plan_load_chunk(ps.chunk, ch + STAGE_WORDS * (size_t)ci);
     if (t < 256) ps.ext[t] = ps.need[t];
+    if (t == 0) ps.top[ci] = 8191;
     __syncthreads();
     for (uint32_t j = t; j < hooked; j += PB) {
       const uint32_t hw = m[128 + j / 2], h = (j & 1) ? hw >> 16 : hw & 0xffffu;
       if ((h >> 8) == (uint32_t)ci && ps.wneed[j]) atomicOr(&ps.ext[h & 255u], ps.wneed[j]);
     }
     __syncthreads();
-    if (t == 0) ps.lv[0] = 0;
-    for (uint32_t M = 1; M <= 4096; M <<= 1) {
+    // the shallowest tree level with a position read from outside: the levels
+    // above it have nothing live (a flat stage has only level 1)
+    if (t < 128 && ps.ext[t]) atomicMin(&ps.top[ci], 32 * t + __ffs(ps.ext[t]) - 1);
+    __syncthreads();
+    uint32_t M0 = 4096;
+    while (M0 > 1 && ps.top[ci] < M0) M0 >>= 1;
+    for (uint32_t c = t; c < M0; c += PB) ps.lv[c] = 0;
+    for (uint32_t M = M0; M <= 4096; M <<= 1) {
       for (uint32_t c = M + t; c < 2 * M; c += PB) {
         uint8_t l = (uint8_t)((ps.ext[c >> 5] >> (c & 31)) & 1u);
-        if (M > 1) {
+        if (M > M0) {
           const uint32_t h = M >> 1;
           const bool is_b = c >= M + h;
           const uint32_t par = is_b ? c - M : c - h;
@@ -276,7 +284,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
         else
           cur[p] = 0;
       }
-      for (uint32_t L = 2048; L; L >>= 1) {
+      for (uint32_t L = 2048; L && 2 * L > ps.top[ci]; L >>= 1) {
         __syncthreads();
         for (uint32_t p = L + t; p < 2 * L; p += PB) {
           if ((ps.live[ci][p >> 5] >> (p & 31)) & 1u)
