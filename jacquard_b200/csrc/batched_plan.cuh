@@ -132,6 +132,9 @@ template <bool X>
 __device__ __forceinline__ uint32_t bp_all(uint32_t e) {
   return e;
 }
+__device__ __forceinline__ uint32_t bp_any_x(uint4 e) { return e.y | e.w; }
+__device__ __forceinline__ uint32_t bp_any_x(uint2 e) { return e.y; }
+__device__ __forceinline__ uint32_t bp_any_x(uint32_t) { return 0; }
 // values written, X words left
 __device__ __forceinline__ void bp_store_values(uint4 *p, uint4 v) {
   uint32_t *w = reinterpret_cast<uint32_t *>(p);
@@ -476,9 +479,11 @@ __global__ void __launch_bounds__(BT, 1)
             const size_t at = (s0 + q) * GS;
             if (cr != 1) {  // not always enabled
               const V en = bp_inv<X>(S[(cr >> 1) * TPE + k], 0u - (cr & 1u));
-              V old = v;
-              if (bp_all<X>(en) != 0xffffffffu) old = __ldcg(vin + at);
-              v = bp_commit<X>(v, old, en);
+              // (every stream enabled: only X enables change the value)
+              if (bp_all<X>(en) != 0xffffffffu)
+                v = bp_commit<X>(v, __ldcg(vin + at), en);
+              else if (X && bp_any_x(en))
+                v = bp_commit<X>(v, v, en);
               if constexpr (TIMED) {
 #pragma unroll
                 for (int j = 0; j < (int)(sizeof(V) / 4 / PV); ++j)
