@@ -126,10 +126,46 @@ struct PlanFetch {
   }
 };
 
-// Gates of an item, one level per CTA barrier; ends with one.  A thread's
-// first gate of a level is loaded before the barrier that opens the level.
-__device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, uint32_t ngr,
-                                           bool isx) {
+// AND of two slot bytes (bit 0 value, bit 1 X).
+template <bool X>
+__device__ __forceinline__ uint32_t plan_and2(uint32_t a, uint32_t b) {
+  return X ? (a & b & 1u) | ((a | b) & (a << 1 | a) & (b << 1 | b) & 2u) : a & b;
+}
+
+// Gates of an item, two logic levels per CTA barrier (plan_build.cuh); ends
+// with one.  A thread's first gate of a phase is loaded before the barrier
+// that opens it.  A phase is latency: two levels in one cost four byte reads
+// a gate instead of two but one chain and one barrier instead of two.
+template <bool X>
+__device__ __forceinline__ void plan_phases(const uint32_t *B, uint8_t *slots, uint32_t ngr) {
+  const uint32_t *ends = B + B[PH_OLEV];
+  const uint2 *gates = reinterpret_cast<const uint2 *>(B + B[PH_OGATE]);
+  const uint32_t nph = B[PH_NLEV];
+  uint8_t *dst = slots + 1 + ngr;
+  uint32_t g = threadIdx.x, g1 = nph ? ends[0] : 0u;
+  uint2 e = g < g1 ? gates[g] : make_uint2(0, 0);
+  __syncthreads();
+  for (uint32_t l = 0; l < nph; ++l) {
+    const uint32_t g2 = l + 1 < nph ? ends[l + 1] : 0u;
+    while (g < g1) {
+      const uint32_t a = slots[(e.x >> 1) & 0x3fffu] ^ (e.x & 1u);
+      const uint32_t b = slots[(e.x >> 16) & 0x3fffu] ^ ((e.x >> 15) & 1u);
+      const uint32_t c = slots[(e.y >> 1) & 0x3fffu] ^ (e.y & 1u);
+      const uint32_t d = slots[(e.y >> 16) & 0x3fffu] ^ ((e.y >> 15) & 1u);
+      dst[g] = (uint8_t)plan_and2<X>(plan_and2<X>(a, b) ^ ((e.x >> 30) & 1u),
+                                     plan_and2<X>(c, d) ^ ((e.y >> 30) & 1u));
+      g += EB;
+      if (g < g1) e = gates[g];
+    }
+    g = g1 + threadIdx.x;
+    g1 = g2;
+    if (g < g1) e = gates[g];
+    __syncthreads();
+  }
+}
+// The same for items listed by level.
+template <bool X>
+__device__ __forceinline__ void plan_levels(const uint32_t *B, uint8_t *slots, uint32_t ngr) {
   const uint32_t *ends = B + B[PH_OLEV], *gates = B + B[PH_OGATE];
   const uint32_t nlev = B[PH_NLEV];
   uint8_t *dst = slots + 1 + ngr;
@@ -141,9 +177,7 @@ __device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, ui
     while (g < g1) {
       const uint32_t a = slots[(e >> 1) & 0x7fffu] ^ (e & 1u);
       const uint32_t b = slots[e >> 17] ^ ((e >> 16) & 1u);
-      uint32_t r = a & b & 1u;
-      if (isx) r |= (a | b) & (a << 1 | a) & (b << 1 | b) & 2u;
-      dst[g] = (uint8_t)r;
+      dst[g] = (uint8_t)plan_and2<X>(a, b);
       g += EB;
       if (g < g1) e = gates[g];
     }
@@ -152,6 +186,13 @@ __device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, ui
     if (g < g1) e = gates[g];
     __syncthreads();
   }
+}
+template <bool X>
+__device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, uint32_t ngr) {
+  if (B[PH_PAIR])
+    plan_phases<X>(B, slots, ngr);
+  else
+    plan_levels<X>(B, slots, ngr);
 }
 
 // SRAM ports of an item: a warp per SRAM, lane = bit of each staged word;
@@ -404,7 +445,7 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
             slots[1 + i] = (uint8_t)(((w.x >> (e & 31)) & 1u) | (isx ? ((w.y >> (e & 31)) & 1u) << 1 : 0u));
           }
         }
-        plan_gates(B, slots, ngr, isx);
+        plan_gates<X>(B, slots, ngr);
         plan_srams(P, B, slots, isx);
         // ---- commit: a warp per writeout word
         {
@@ -577,7 +618,7 @@ __global__ void __launch_bounds__(EB, 1) plan_mirror_kernel(const __grid_constan
             }
           }
         }
-        plan_gates(B, slots, ngr, isx);
+        plan_gates<X>(B, slots, ngr);
         plan_srams(P, B, slots, isx);
         // ---- commit: a warp per writeout word, to the snapshot and to every
         // CTA's mirror

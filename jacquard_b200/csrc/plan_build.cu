@@ -33,7 +33,7 @@ struct PlanShared {
   uint32_t lev[PLAN_MAX_LEVELS], lev_base[PLAN_MAX_LEVELS];
   uint32_t warp_sum[32];
   int bad;
-  uint32_t max_lev, n_gates;
+  uint32_t max_lev, n_gates, pair;
   unsigned long long off;
 };
 
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   };
   // ---- forward over the stages: reference of every live position; with
   // `gates` the gates are written, else counted per level
-  auto forward = [&](uint32_t *gates, uint32_t gate0) {
+  auto forward = [&](uint32_t *gates, uint32_t gate0, bool pair) {
     uint32_t *prev = ps.ref_a, *cur = ps.ref_b;
     for (uint32_t ci = 0; ci < ns; ++ci) {
       plan_load_chunk(ps.chunk, ch + STAGE_WORDS * (size_t)ci);
@@ -266,10 +266,26 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
         if (plan_and(a, b, plan_flag(ps.chunk, p, 0), plan_flag(ps.chunk, p, 1),
                      plan_flag(ps.chunk, p, 2), r, ra, rb)) {
           const uint32_t l = r < PLAN_MAX_LEVELS ? r : PLAN_MAX_LEVELS - 1;
-          const uint32_t k = atomicAdd(&ps.lev[l], 1u);
+          const uint32_t ph = pair && gates ? (l + 1) / 2 : l;  // its phase
+          const uint32_t k = atomicAdd(&ps.lev[ph], 1u);
           if (gates) {
-            const uint32_t g = ps.lev_base[l] + k;
-            gates[g] = (ra & 0xffffu) | (rb << 16);
+            const uint32_t g = ps.lev_base[ph] + k;
+            if (!pair) {
+              gates[g] = (ra & 0xffffu) | (rb << 16);
+            } else {
+              // an operand of an even level: a gate of the odd level before it
+              // by its own operands, anything else as (it AND 1)
+              auto half = [&](uint32_t o) -> uint32_t {
+                if (!(l & 1) && (o >> 16) == l - 1)
+                  return gates[2 * (((o >> 1) & 0x7fffu) - gate0)] | ((o & 1u) << 30);
+                return (o & 0x7fffu) | (1u << 15);
+              };
+              const bool odd = l & 1;
+              const uint32_t x = odd ? (ra & 0x7fffu) | ((rb & 0x7fffu) << 15) : half(ra);
+              const uint32_t y = odd ? 1u | (1u << 15) : half(rb);
+              gates[2 * g] = x;
+              gates[2 * g + 1] = y;
+            }
             r = (l << 16) | ((gate0 + g) << 1);
           } else {
             r = (l << 16) | (1u << 1);
@@ -308,24 +324,37 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   gr_refs();
   for (uint32_t l = t; l < PLAN_MAX_LEVELS; l += PB) ps.lev[l] = 0;
   __syncthreads();
-  forward(nullptr, 0);
+  forward(nullptr, 0, false);
   if (t == 0) {
     uint32_t n = 0, top = 0;
     for (uint32_t l = 1; l < PLAN_MAX_LEVELS; ++l) {
-      ps.lev_base[l] = n;
       n += ps.lev[l];
       if (ps.lev[l]) top = l;
     }
     ps.n_gates = n;
-    ps.max_lev = top;
     if (ps.lev[PLAN_MAX_LEVELS - 1]) ps.bad = 1;  // deeper levels share the last count
+    // pairs of levels where levels are small (PLAN_PAIR_GATES)
+    ps.pair = P.mode != PLAN_SIGNALS && n <= PLAN_PAIR_GATES * top &&
+              1 + n_gr + n + 32 * nsr <= PLAN_MAX_SLOTS / 2;
+    if (ps.pair) {
+      top = (top + 1) / 2;
+      for (uint32_t l = 1; l <= top; ++l) ps.lev[l] = ps.lev[2 * l - 1] + ps.lev[2 * l];
+    }
+    ps.max_lev = top;
+    n = 0;
+    for (uint32_t l = 1; l <= top; ++l) {
+      ps.lev_base[l] = n;
+      n += ps.lev[l];
+    }
   }
   __syncthreads();
+  const bool pair = ps.pair;
   const uint32_t n_gates = ps.n_gates, n_lev = ps.max_lev, nw = j1 - j0;
   const uint32_t gate0 = 1 + n_gr, sr_slot = gate0 + n_gates, n_slots = sr_slot + 32 * nsr;
   auto al = [](uint32_t w) { return (w + 3u) & ~3u; };
   const uint32_t o_gw = PH_SIZE, o_exp = o_gw + (P.mode == PLAN_WORDS ? al(n_gw) : 0u), o_lev = o_exp + al(n_gr),
-                 o_gate = o_lev + al(n_lev), o_sram = o_gate + al(n_gates),
+                 o_gate = o_lev + al(n_lev),
+                 o_sram = o_gate + al(pair ? 2 * n_gates : n_gates),
                  o_com = o_sram + 96 * nsr, o_keep = o_com + 32 * nw, words = o_keep + al(nw);
   if (n_slots > PLAN_MAX_SLOTS) bad = true;
   if (__syncthreads_or(bad || ps.bad)) {
@@ -426,7 +455,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   gr_refs();
   for (uint32_t l = t; l < PLAN_MAX_LEVELS; l += PB) ps.lev[l] = 0;
   __syncthreads();
-  forward(B + o_gate, gate0);
+  forward(B + o_gate, gate0, pair);
   for (uint32_t l = t; l < n_lev; l += PB) B[o_lev + l] = ps.lev_base[1 + l] + ps.lev[1 + l];
   // ---- SRAM ports, then the commit: references of the staged words and of
   // each own writeout bit and its clock enable
@@ -473,6 +502,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     B[PH_OKEEP] = o_keep;
     B[PH_SRSLOT] = sr_slot;
     B[PH_PART] = pid;
+    B[PH_PAIR] = pair;
   }
 }
 
@@ -574,7 +604,7 @@ size_t plan_workspace_words(size_t blocks_data_len, size_t num_blocks, size_t nm
   const size_t entries = num_blocks * nms;
   const size_t parts = blocks_data_len / PLAN_MIN_PART + 1;
   return PlanLayout(entries, parts, parts + nms * PLAN_SPARE_ITEMS, state_words).blob +
-         blocks_data_len / 2 + 4096;
+         blocks_data_len + nms * PLAN_SPARE_ITEMS * 1024 + 4096;
 }
 
 size_t plan_smem_limit(const void *fn) {

@@ -29,12 +29,23 @@ enum PlanMode : uint32_t {
   PLAN_MIRROR,   // (state word, bit) per slot
   PLAN_SIGNALS,  // a signal per slot (batched form)
 };
+// Gates: one word per gate, its operand references, by logic level; or, in
+// items of the one-stream forms whose levels average at most PLAN_PAIR_GATES
+// gates, two words per gate by pair of levels (a phase).  There each half is
+// an operand as the AND of two references x | y << 15 (14-bit slots), inverted
+// by bit 30: a gate of an even level names the operands of the odd level
+// before it instead of its slot, so a phase needs no barrier inside.  Small
+// levels are latency (16k gates, 8 levels of about 300 gates per item: 2.36 us
+// a stage by level, 2.10 by pair; 256k gates 2.52 / 2.43), large ones the byte
+// reads of shared memory, which pairs double (2M gates, levels of about 500:
+// 4.13 / 4.27).
+constexpr uint32_t PLAN_PAIR_GATES = 400;
 
 // Item header (words of the item's blob; section offsets in words, 16-byte
 // aligned).
 enum PlanHdr : uint32_t {
   PH_WORDS, PH_NGW, PH_NGR, PH_NLEV, PH_NW, PH_IO, PH_NSR, PH_SRAM_OFF, PH_ISX, PH_XOFF,
-  PH_OGW, PH_OEXP, PH_OLEV, PH_OGATE, PH_OSRAM, PH_OCOM, PH_OKEEP, PH_SRSLOT, PH_PART, PH_SIZE = 20
+  PH_OGW, PH_OEXP, PH_OLEV, PH_OGATE, PH_OSRAM, PH_OCOM, PH_OKEEP, PH_SRSLOT, PH_PART, PH_PAIR, PH_SIZE = 20
 };
 
 // Build result: unsupported flag (bit 0: the plan, bit 1: its mirrored form),
