@@ -164,6 +164,7 @@ typedef struct {
   uint32_t max_blob, max_slots, max_gw; /* largest item */
   uint32_t stage_item[33];              /* first item of each major stage */
   uint32_t widest, nbuf;                /* most items of a stage, blob buffers */
+  uint32_t paired;                      /* two logic levels per step in every item */
   /* form that keeps the snapshot in the shared memory of one cluster */
   uint32_t mirrored, rio, xoff, n_unwritten, stage_words[32];
   const uint32_t *unwritten;
@@ -331,7 +332,7 @@ typedef struct {
   size_t num_major_stages, num_partitions;
   uint32_t lanes, lanes_per_item;
   int32_t x_interleaved;
-  uint32_t with_x, supported;
+  uint32_t with_x, supported, paired; /* paired: two logic levels per step */
   uint32_t max_blob, max_slots, nbuf; /* largest item, blob buffers */
   uint32_t widest, stage_item[33];    /* most items of a stage, first of each */
   size_t used_words;

@@ -38,7 +38,7 @@ class BatchedPlan(ctypes.Structure):
                 ("lanes", ctypes.c_uint32),
                 ("lanes_per_item", ctypes.c_uint32), ("x_interleaved", ctypes.c_int32),
                 ("with_x", ctypes.c_uint32), ("supported", ctypes.c_uint32),
-                ("max_blob", ctypes.c_uint32), ("max_slots", ctypes.c_uint32),
+                ("paired", ctypes.c_uint32), ("max_blob", ctypes.c_uint32), ("max_slots", ctypes.c_uint32),
                 ("nbuf", ctypes.c_uint32), ("widest", ctypes.c_uint32),
                 ("stage_item", ctypes.c_uint32 * 33), ("used_words", ctypes.c_size_t),
                 ("blob", vp), ("item_off", vp), ("item_words", vp)]

@@ -14,6 +14,16 @@
 
 namespace jqk {
 
+// Gates of a level up to which a script's items take two levels per barrier:
+// half a round of the CTA (512 threads, 16 bytes of a slot each), so that a
+// pair of levels is one round.  All of a plan's items or none, so that the
+// kernel has one of the two loops: with both, items that do not use the second
+// ran 1 to 2.5% slower.  16k gates x 32 streams 908 / 812 us a pass, 256k x 64
+// 1950 / 1815, 16k x 256 (octets, levels of 16) 526 / 497.
+constexpr uint32_t bplan_pair_gates(uint32_t lw, bool x) {
+  return lw == 8 ? (x ? 64 : 128) : 256;
+}
+
 struct BPlanParams {
   const uint32_t *blob;
   const unsigned long long *item_off;
@@ -233,7 +243,7 @@ __device__ __noinline__ void bp_io(const BatchParams &P, const uint32_t *in, uin
   }
 }
 
-template <int LW, bool X, bool TIMED>
+template <int LW, bool X, bool TIMED, bool PAIR>
 __global__ void __launch_bounds__(BT, 1)
     jq_bplan_kernel(const __grid_constant__ BatchParams P, const __grid_constant__ BPlanParams Q) {
   using V = typename LaneVec<LW, X>::T;
@@ -405,7 +415,7 @@ __global__ void __launch_bounds__(BT, 1)
         if (sizeof(V) == 16) asm volatile("cp.async.wait_all;" ::: "memory");
         // ---- gates, one level per CTA barrier; a thread's first gate of a
         // level is loaded before the barrier that opens the level
-        {
+        if constexpr (!PAIR) {
           const uint32_t *ends = B + B[PH_OLEV], *gates = B + B[PH_OGATE];
           const uint32_t nlev = B[PH_NLEV];
           V *dst = S + (1 + ngr) * TPE + k;
@@ -419,6 +429,35 @@ __global__ void __launch_bounds__(BT, 1)
               const V a = S[((e >> 1) & 0x7fffu) * TPE + k], b = S[(e >> 17) * TPE + k];
               dst[g * TPE] = bp_and<X>(bp_inv<X>(a, 0u - (e & 1u)),
                                        bp_inv<X>(b, 0u - ((e >> 16) & 1u)));
+              g += NE;
+              if (g < g1) e = gates[g];
+            }
+            g = g1 + el;
+            g1 = g2;
+            if (g < g1) e = gates[g];
+            __syncthreads();
+          }
+        }
+        else {
+          // two levels per barrier (plan_build.cuh)
+          const uint32_t *ends = B + B[PH_OLEV];
+          const uint2 *gates = reinterpret_cast<const uint2 *>(B + B[PH_OGATE]);
+          const uint32_t nph = B[PH_NLEV];
+          V *dst = S + (1 + ngr) * TPE + k;
+          uint32_t g = el, g1 = nph ? ends[0] : 0u;
+          uint2 e = g < g1 ? gates[g] : make_uint2(0, 0);
+          __syncthreads();
+          for (uint32_t l = 0; l < nph; ++l) {
+            const uint32_t g2 = l + 1 < nph ? ends[l + 1] : 0u;
+#pragma unroll 1
+            while (g < g1) {
+              auto half = [&](uint32_t h) {
+                const V x = S[((h >> 1) & 0x3fffu) * TPE + k], y = S[((h >> 16) & 0x3fffu) * TPE + k];
+                return bp_inv<X>(bp_and<X>(bp_inv<X>(x, 0u - (h & 1u)),
+                                           bp_inv<X>(y, 0u - ((h >> 15) & 1u))),
+                                 0u - ((h >> 30) & 1u));
+              };
+              dst[g * TPE] = bp_and<X>(half(e.x), half(e.y));
               g += NE;
               if (g < g1) e = gates[g];
             }

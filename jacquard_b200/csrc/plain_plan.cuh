@@ -187,9 +187,11 @@ __device__ __forceinline__ void plan_levels(const uint32_t *B, uint8_t *slots, u
     __syncthreads();
   }
 }
-template <bool X>
+// PAIRS: every item of the plan is listed by pairs, so the kernel has one loop
+// (small design 555 us a pass with both, 537 with one).
+template <bool X, bool PAIRS>
 __device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, uint32_t ngr) {
-  if (B[PH_PAIR])
+  if (PAIRS || B[PH_PAIR])
     plan_phases<X>(B, slots, ngr);
   else
     plan_levels<X>(B, slots, ngr);
@@ -297,7 +299,7 @@ __device__ __forceinline__ uint2 plan_poll(const uint2 *p) {
 // 128 items a stage, per major stage: 4.76 us without, 4.33 / 4.21 / 4.14
 // with slack 1 / 4 / 16; 48 items: 2.50 us without, 2.72 with, so those run
 // without.  A grid barrier with a release fence instead took 4.39 and 3.33 us.
-template <bool X>
+template <bool X, bool PAIRS>
 __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant__ PlanParams P) {
   extern __shared__ __align__(128) uint8_t dyn[];
   __shared__ uint64_t bar[2];
@@ -445,7 +447,7 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
             slots[1 + i] = (uint8_t)(((w.x >> (e & 31)) & 1u) | (isx ? ((w.y >> (e & 31)) & 1u) << 1 : 0u));
           }
         }
-        plan_gates<X>(B, slots, ngr);
+        plan_gates<X, PAIRS>(B, slots, ngr);
         plan_srams(P, B, slots, isx);
         // ---- commit: a warp per writeout word
         {
@@ -507,7 +509,7 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
 // two mbarriers, for even and odd cycles, and neither sees the bytes of two
 // phases at once.  Words of snapshot c + 2 overwrite those of c only after
 // the last item that reads snapshot c has sent its own.
-template <bool X>
+template <bool X, bool PAIRS>
 __global__ void __launch_bounds__(EB, 1) plan_mirror_kernel(const __grid_constant__ PlanParams P) {
   extern __shared__ __align__(128) uint8_t dyn[];
   __shared__ uint64_t bar[2], stage_bar[64];  // stage_bar[2 ms + cycle parity]
@@ -618,7 +620,7 @@ __global__ void __launch_bounds__(EB, 1) plan_mirror_kernel(const __grid_constan
             }
           }
         }
-        plan_gates<X>(B, slots, ngr);
+        plan_gates<X, PAIRS>(B, slots, ngr);
         plan_srams(P, B, slots, isx);
         // ---- commit: a warp per writeout word, to the snapshot and to every
         // CTA's mirror

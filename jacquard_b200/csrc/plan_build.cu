@@ -15,6 +15,7 @@ struct PlanBuildParams {
   const uint32_t *writer;              // per state word: major stage + 1 that writes it, or 0
   uint32_t writer_words;
   uint32_t mode;                       // PlanMode
+  uint32_t pair_gates;                 // gates a level up to which levels go in pairs
   uint32_t *blob;
   unsigned long long blob_cap;
   unsigned long long *item_off;        // per item: blob word offset
@@ -333,9 +334,11 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     }
     ps.n_gates = n;
     if (ps.lev[PLAN_MAX_LEVELS - 1]) ps.bad = 1;  // deeper levels share the last count
-    // pairs of levels where levels are small (PLAN_PAIR_GATES)
-    ps.pair = P.mode != PLAN_SIGNALS && n <= PLAN_PAIR_GATES * top &&
+    // pairs of levels where levels are small
+    ps.pair = n <= (uint64_t)P.pair_gates * top &&
               1 + n_gr + n + 32 * nsr <= PLAN_MAX_SLOTS / 2;
+    if (top) atomicMax(&P.res->max_level, (n + top - 1) / top);
+    if (!ps.pair) atomicOr(&P.res->unpaired, 1u);
     if (ps.pair) {
       top = (top + 1) / 2;
       for (uint32_t l = 1; l <= top; ++l) ps.lev[l] = ps.lev[2 * l - 1] + ps.lev[2 * l];
@@ -668,7 +671,7 @@ int PlanBuilder::scan(bool *ok) {
   return JQ_OK;
 }
 
-int PlanBuilder::build(PlanMode mode, size_t want, size_t round, bool *ok) {
+int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok) {
   *ok = false;
   const size_t entries = num_blocks * nms;
   std::vector<uint32_t> items;
@@ -698,7 +701,7 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, bool *ok) {
   PlanResult *res = reinterpret_cast<PlanResult *>(ws);
   r.unsupported = 0;
   r.used = 0;
-  r.max_blob = r.max_slots = r.max_gw = 0;
+  r.max_blob = r.max_slots = r.max_gw = r.max_level = r.unpaired = 0;
   if (cudaMemcpyAsync(res, &r, sizeof r, cudaMemcpyHostToDevice, st) != cudaSuccess ||
       cudaMemcpyAsync(ws + lay.items, items.data(), items.size() * 4, cudaMemcpyHostToDevice,
                       st) != cudaSuccess)
@@ -711,6 +714,7 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, bool *ok) {
   B.writer = ws + lay.writer;
   B.writer_words = (uint32_t)state_words;
   B.mode = mode;
+  B.pair_gates = pair_gates;
   B.blob = ws + lay.blob;
   B.blob_cap = ws_words - lay.blob;
   B.item_off = reinterpret_cast<unsigned long long *>(ws + lay.item_off);

@@ -30,16 +30,11 @@ enum PlanMode : uint32_t {
   PLAN_SIGNALS,  // a signal per slot (batched form)
 };
 // Gates: one word per gate, its operand references, by logic level; or, in
-// items of the one-stream forms whose levels average at most PLAN_PAIR_GATES
-// gates, two words per gate by pair of levels (a phase).  There each half is
-// an operand as the AND of two references x | y << 15 (14-bit slots), inverted
-// by bit 30: a gate of an even level names the operands of the odd level
-// before it instead of its slot, so a phase needs no barrier inside.  Small
-// levels are latency (16k gates, 8 levels of about 300 gates per item: 2.36 us
-// a stage by level, 2.10 by pair; 256k gates 2.52 / 2.43), large ones the byte
-// reads of shared memory, which pairs double (2M gates, levels of about 500:
-// 4.13 / 4.27).
-constexpr uint32_t PLAN_PAIR_GATES = 400;
+// items of small levels (PH_PAIR; the caller of the build sets how small), two
+// words per gate by pair of levels (a phase).  There each half is an operand
+// as the AND of two references x | y << 15 (14-bit slots), inverted by bit 30:
+// a gate of an even level names the operands of the odd level before it
+// instead of its slot, so a phase needs no barrier inside.
 
 // Item header (words of the item's blob; section offsets in words, 16-byte
 // aligned).
@@ -57,7 +52,9 @@ struct PlanResult {
   uint32_t unsupported, x_use;
   unsigned long long used;
   uint32_t max_blob, max_slots, max_gw, rio;
-  uint32_t xoff_max, xoff_inv_max, n_unwritten, pad;
+  uint32_t xoff_max, xoff_inv_max, n_unwritten;
+  uint32_t max_level;     // most gates per level of any item, on average
+  uint32_t unpaired, pad;  // an item lists its gates by level
   uint32_t stage_words[32];
 };
 
@@ -87,8 +84,9 @@ struct PlanBuilder {
   const uint32_t *unwritten() const;
   // Items: every partition of stage ms split towards want / per_stage[ms]
   // ways.  With `round` (items a stage runs at a time) a stage's items are put
-  // by decreasing size, every second round reversed.
-  int build(PlanMode mode, size_t want, size_t round, bool *ok);
+  // by decreasing size, every second round reversed.  Items whose levels
+  // average at most pair_gates gates list them by pair of levels.
+  int build(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok);
 };
 
 // Words of workspace a build of any script of this size fits in.

@@ -2641,16 +2641,21 @@ int jq_simulate_batched(const jq_batch_args *a) {
 // ---- gate-list plan (batched_plan.cuh)
 
 extern "C++" {
-template <bool X, bool TIMED>
+template <bool X, bool TIMED, bool PAIR>
 static const void *bplan_fn_of(uint32_t lw) {
-  return lw == 8   ? (const void *)jq_bplan_kernel<8, X, TIMED>
-         : lw == 2 ? (const void *)jq_bplan_kernel<2, X, TIMED>
-                   : (const void *)jq_bplan_kernel<1, X, TIMED>;
+  return lw == 8   ? (const void *)jq_bplan_kernel<8, X, TIMED, PAIR>
+         : lw == 2 ? (const void *)jq_bplan_kernel<2, X, TIMED, PAIR>
+                   : (const void *)jq_bplan_kernel<1, X, TIMED, PAIR>;
+}
+template <bool X>
+static const void *bplan_fn_of(uint32_t lw, bool timed, bool pair) {
+  if (timed) return pair ? bplan_fn_of<X, true, true>(lw) : bplan_fn_of<X, true, false>(lw);
+  return pair ? bplan_fn_of<X, false, true>(lw) : bplan_fn_of<X, false, false>(lw);
 }
 }
-static const void *bplan_fn(uint32_t lw, bool x, bool timed) {
-  if (timed) return x ? bplan_fn_of<true, true>(lw) : bplan_fn_of<false, true>(lw);
-  return x ? bplan_fn_of<true, false>(lw) : bplan_fn_of<false, false>(lw);
+static const void *bplan_fn(const jq_batched_plan *p, bool timed) {
+  return p->with_x ? bplan_fn_of<true>(p->lanes_per_item, timed, p->paired)
+                   : bplan_fn_of<false>(p->lanes_per_item, timed, p->paired);
 }
 
 static size_t bplan_smem(const jq_batched_plan *p, uint32_t nbuf) {
@@ -2694,12 +2699,15 @@ int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_dat
   if ((b.r.x_use & 2u) && (!x || b.r.xoff_max != state_words)) return JQ_OK;
   const size_t groups = lanes / lanes_per_item;
   const size_t round = (size_t)sms > groups ? (size_t)sms / groups : 1;
-  const size_t lim = plan_smem_limit(bplan_fn(lanes_per_item, x, true));
+  const size_t lim = plan_smem_limit(bplan_fn(plan, true));
   // one item per CTA where a stage has few partitions, more parts where an
   // item's slots do not fit
-  for (size_t want = round;; want *= 2) {
-    rc = b.build(PLAN_SIGNALS, want, round, &ok);
+  const uint32_t pair_gates = bplan_pair_gates(lanes_per_item, x);
+  bool pairs = true;
+  for (size_t want = round;;) {
+    rc = b.build(PLAN_SIGNALS, want, round, plan->paired ? 0xffffffffu : 0u, &ok);
     if (rc != JQ_OK) return rc;
+    plan->supported = 0;
     if (ok) {
       plan->max_blob = b.r.max_blob;
       plan->max_slots = b.r.max_slots;
@@ -2712,7 +2720,19 @@ int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_dat
       plan->item_words = b.item_words;
       plan->supported = plan->nbuf != 0;
     }
-    if (plan->supported || want >= PLAN_MAX_NSUB * b.most) return JQ_OK;
+    if (plan->supported && (plan->paired || !pairs || b.r.max_level > pair_gates ||
+                            plan->max_slots > PLAN_MAX_SLOTS / 2))
+      return JQ_OK;
+    if (plan->supported) {  // small levels throughout: once more, by pairs
+      plan->paired = 1;
+    } else if (plan->paired) {  // its gates take more room than there is: by levels
+      plan->paired = 0;
+      pairs = false;
+    } else if (want >= PLAN_MAX_NSUB * b.most) {
+      return JQ_OK;
+    } else {
+      want *= 2;
+    }
   }
 }
 
@@ -2741,7 +2761,7 @@ int jq_simulate_batched_planned(const jq_batch_args *a, const jq_batched_plan *p
   P.slot = launch_slot(a->stream, true);
   if (P.slot < 0) return JQ_ERR_TOO_MANY_STREAMS;
   cudaStream_t st = (cudaStream_t)a->stream;
-  const void *fn = bplan_fn(p->lanes_per_item, p->with_x, P.constraints != nullptr);
+  const void *fn = bplan_fn(p, P.constraints != nullptr);
   const int smem = (int)bplan_smem(p, p->nbuf);
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
     return JQ_ERR_LAUNCH;

@@ -507,6 +507,11 @@ constexpr uint32_t PLAN_CLUSTER = 16;
 constexpr size_t PLAN_MIRROR_PARTS = 2;
 constexpr size_t PLAN_MIRROR_BYTES = 112 * 1024;
 constexpr uint32_t PLAN_HINT_ITEMS = 64, PLAN_HINT_SLACK = 16;
+// Gates of a level up to which an item takes two levels per barrier.  Small
+// levels are latency (16k gates, 8 levels of about 300 per item: 2.36 us a stage
+// by level, 2.17 by pair; 256k gates 2.52 / 2.43), large ones the byte reads,
+// which pairs double (2M gates, levels of about 500: 4.13 / 4.27).
+constexpr uint32_t PLAN_PAIR_GATES = 400;
 constexpr uint32_t PLAN_GRID_ONLY = 0xffffffffu;  // target_items: never the mirrored form
 
 // Shared memory of the executor: blob buffers and slots, then the state
@@ -517,11 +522,14 @@ size_t plan_smem_bytes(const jq_plain_plan *p, uint32_t nbuf) {
                              : 8 * (size_t)((p->max_gw + 1) & ~1u) + 2 * 8 * 256);
 }
 
+template <bool X, bool PAIRS>
+const void *plan_fn_of(const jq_plain_plan *p) {
+  return p->mirrored ? (const void *)plan_mirror_kernel<X, PAIRS>
+                     : (const void *)plan_flow_kernel<X, PAIRS>;
+}
 const void *plan_fn(const jq_plain_plan *p) {
-  if (p->mirrored)
-    return p->xoff ? (const void *)plan_mirror_kernel<true>
-                   : (const void *)plan_mirror_kernel<false>;
-  return p->xoff ? (const void *)plan_flow_kernel<true> : (const void *)plan_flow_kernel<false>;
+  if (p->xoff) return p->paired ? plan_fn_of<true, true>(p) : plan_fn_of<true, false>(p);
+  return p->paired ? plan_fn_of<false, true>(p) : plan_fn_of<false, false>(p);
 }
 
 // Launch of the mirrored form: one cluster of the next power of two CTAs.
@@ -577,10 +585,11 @@ int plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t n
     const size_t want = target && target != PLAN_GRID_ONLY ? target
                         : mirrored                         ? PLAN_CLUSTER
                                                            : PLAN_GRID_ITEMS;
-    rc = b.build(mirrored ? PLAN_MIRROR : PLAN_WORDS, want, 0, &ok);
+    rc = b.build(mirrored ? PLAN_MIRROR : PLAN_WORDS, want, 0, PLAN_PAIR_GATES, &ok);
     if (rc != JQ_OK) return rc;
     if (ok) {
       plan->mirrored = mirrored;
+      plan->paired = !b.r.unpaired;
       plan->exchange_words = mirrored ? 0 : 4 * (size_t)b.r.rio * (plan->xoff ? 4 : 2);
       plan->max_blob = b.r.max_blob;
       plan->max_slots = b.r.max_slots;

@@ -30,7 +30,7 @@ class PlainPlan(ctypes.Structure):
                 ("supported", ctypes.c_uint32), ("max_blob", ctypes.c_uint32),
                 ("max_slots", ctypes.c_uint32), ("max_gw", ctypes.c_uint32),
                 ("stage_item", ctypes.c_uint32 * 33), ("widest", ctypes.c_uint32),
-                ("nbuf", ctypes.c_uint32), ("mirrored", ctypes.c_uint32), ("rio", ctypes.c_uint32),
+                ("nbuf", ctypes.c_uint32), ("paired", ctypes.c_uint32), ("mirrored", ctypes.c_uint32), ("rio", ctypes.c_uint32),
                 ("xoff", ctypes.c_uint32), ("n_unwritten", ctypes.c_uint32),
                 ("stage_words", ctypes.c_uint32 * 32), ("unwritten", vp),
                 ("exchange_words", ctypes.c_size_t), ("used_words", ctypes.c_size_t),
