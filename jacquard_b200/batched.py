@@ -223,17 +223,28 @@ class BatchedSim:
                 raise ValueError(f"octet items need an X-propagating script, lanes divisible by 8 "
                                  f"and every partition within {cap} slots (needs {need:#x})")
             self.x_interleaved = 2
-        # the gate-list plan in the items asked for, or the widest that the
-        # lanes divide into; without one the prepared script runs
+        # The gate-list plan in the items asked for, else octets where they
+        # occupy two thirds of the SMs, lane pairs or single lanes where not
+        # (8 lane words of a 256k-gate design, us per pass octets / pairs: 48
+        # octet items a stage 736 / 585, 96 713 / 683, 144 788 / 881); without
+        # a plan the prepared script runs.
         self.plan = self._plan_ws = None
         if planned and wo_slots is None:
-            forms = [w for w in (8, 2, 1) if lanes % w == 0 and lanes_per_item in (0, w)]
-            for w in forms:
+            sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+            octets = None
+            for w in [w for w in (8, 2, 1) if lanes % w == 0 and lanes_per_item in (0, w)]:
                 layout = (2 if script.xprop_enabled else 3) if w == 8 else \
                     (1 if script.xprop_enabled else 0)
-                if self._build_plan(w, layout):
-                    self.x_interleaved = layout
-                    break
+                if not self._build_plan(w, layout):
+                    continue
+                self.x_interleaved = layout
+                if w == 8 and not lanes_per_item and 3 * self.plan.widest * (lanes // 8) < 2 * sms:
+                    octets = (self.plan, self._plan_ws, layout)
+                    self.plan = None
+                    continue
+                break
+            if self.plan is None and octets is not None:
+                self.plan, self._plan_ws, self.x_interleaved = octets
         if self.plan is None:
             self._prepared()
         regions = getattr(script, "input_regions", None)

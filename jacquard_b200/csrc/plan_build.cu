@@ -100,8 +100,10 @@ __device__ __forceinline__ bool plan_and(uint32_t a, uint32_t b, uint32_t xa, ui
 }
 
 // One CTA builds one item: partition `items[2i]`, writeout slots
-// [nio * sub / nsub, nio * (sub + 1) / nsub) (partitions with SRAMs have one
-// item).  The result's `unsupported` flag is set for what the plan does not
+// [nio * sub / nsub, nio * (sub + 1) / nsub); of a partition with SRAMs the
+// last item has the ports, the duplicate and the SRAM slots, the others share
+// the hooked slots (flag bit 2 when one of them reads an SRAM's output).  The
+// result's `unsupported` flag is set for what the plan does not
 // represent -- a writeout slot that no hook, SRAM or duplicate writes, or a
 // permutation that reads one an earlier partition left (both observe the
 // per-block arrays of the script kernel), a partition that reads what the
@@ -119,14 +121,21 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
                  ndup = m[7], isx = m[8], xoff = m[9];
   const uint32_t my_ms = P.part_ms[pid];
   bool bad = ns > PLAN_MAX_NS || nio > 256 || nsr * 4 + ndup > 256 || nsr + ndup > nio ||
-             (nsr && nsub > 1) || R > 32;
+             R > 32;
   if (bad) {  // uniform
     if (t == 0) atomicOr(&P.res->unsupported, 1u);
     return;
   }
   const uint32_t *gr = m + 256, *ch = gr + 512 * (size_t)R;
-  const uint32_t j0 = nio * sub / nsub, j1 = nio * (sub + 1) / nsub;
   const uint32_t hooked = nio - nsr - ndup;  // slots below are hooked
+  uint32_t j0 = nio * sub / nsub, j1 = nio * (sub + 1) / nsub;
+  uint32_t ports = nsr;  // SRAM ports of this item: of a split partition's last item
+  if (nsr && nsub > 1) {
+    const bool last = sub + 1 == nsub;
+    j0 = last ? hooked : hooked * sub / (nsub - 1);
+    j1 = last ? nio : hooked * (sub + 1) / (nsub - 1);
+    ports = last ? nsr : 0;
+  }
   if (t == 0) ps.bad = 0;
   if (t < 256) {
     ps.wneed[t] = t >= j0 && t < j1 ? 0xffffffffu : 0u;
@@ -143,11 +152,18 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
       else atomicOr(&ps.wneed[p >> 5], 1u << (p & 31));
     }
   __syncthreads();
+  // an item without the ports cannot read what they read
+  bool no_port = false;
+  for (uint32_t j = hooked + ndup + t; j < nio; j += PB) no_port |= !ports && ps.wneed[j] != 0;
+  if (__syncthreads_or(no_port)) {
+    if (t == 0) atomicOr(&P.res->unsupported, 4u);
+    return;
+  }
   plan_load_chunk(ps.chunk, ch + STAGE_WORDS * (size_t)ns);
   for (uint32_t q = t; q < (nsr * 4 + ndup) * 32; q += PB) {
     bool use;
     if (q < nsr * 128) {
-      use = (q & 127u) < 96u;
+      use = ports && (q & 127u) < 96u;
     } else {
       const uint32_t k = (q >> 5) - nsr * 4;  // duplicate k, slot hooked + k
       use = (ps.wneed[hooked + k] >> (q & 31)) & 1u;
@@ -336,7 +352,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     if (ps.lev[PLAN_MAX_LEVELS - 1]) ps.bad = 1;  // deeper levels share the last count
     // pairs of levels where levels are small
     ps.pair = n <= (uint64_t)P.pair_gates * top &&
-              1 + n_gr + n + 32 * nsr <= PLAN_MAX_SLOTS / 2;
+              1 + n_gr + n + 32 * ports <= PLAN_MAX_SLOTS / 2;
     if (top) atomicMax(&P.res->max_level, (n + top - 1) / top);
     if (!ps.pair) atomicOr(&P.res->unpaired, 1u);
     if (ps.pair) {
@@ -353,12 +369,12 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   __syncthreads();
   const bool pair = ps.pair;
   const uint32_t n_gates = ps.n_gates, n_lev = ps.max_lev, nw = j1 - j0;
-  const uint32_t gate0 = 1 + n_gr, sr_slot = gate0 + n_gates, n_slots = sr_slot + 32 * nsr;
+  const uint32_t gate0 = 1 + n_gr, sr_slot = gate0 + n_gates, n_slots = sr_slot + 32 * ports;
   auto al = [](uint32_t w) { return (w + 3u) & ~3u; };
   const uint32_t o_gw = PH_SIZE, o_exp = o_gw + (P.mode == PLAN_WORDS ? al(n_gw) : 0u), o_lev = o_exp + al(n_gr),
                  o_gate = o_lev + al(n_lev),
                  o_sram = o_gate + al(pair ? 2 * n_gates : n_gates),
-                 o_com = o_sram + 96 * nsr, o_keep = o_com + 32 * nw, words = o_keep + al(nw);
+                 o_com = o_sram + 96 * ports, o_keep = o_com + 32 * nw, words = o_keep + al(nw);
   if (n_slots > PLAN_MAX_SLOTS) bad = true;
   if (__syncthreads_or(bad || ps.bad)) {
     if (t == 0) atomicOr(&P.res->unsupported, 1u);
@@ -467,12 +483,12 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     const uint32_t inv = plan_flag(ps.chunk, q, 0);
     return plan_flag(ps.chunk, q, 1) ? inv : ps.woref[plan_perm(ps.chunk, q)] ^ inv;
   };
-  for (uint32_t i = t; i < 96 * nsr; i += PB) B[o_sram + i] = staged(128 * (i / 96) + i % 96);
+  for (uint32_t i = t; i < 96 * ports; i += PB) B[o_sram + i] = staged(128 * (i / 96) + i % 96);
   // duplicate and SRAM slots get their references too
   for (uint32_t q = t; q < 32 * ndup; q += PB)
     if ((ps.wneed[hooked + (q >> 5)] >> (q & 31)) & 1u)
       ps.woref[32 * hooked + q] = (uint16_t)staged(nsr * 128 + q);
-  for (uint32_t q = t; q < 32 * nsr; q += PB)
+  for (uint32_t q = t; q < 32 * ports; q += PB)
     ps.woref[32 * (hooked + ndup) + q] = (uint16_t)((sr_slot + q) << 1);
   __syncthreads();
   plan_load_chunk(ps.chunk, ch + STAGE_WORDS * (size_t)(ns + 1));
@@ -492,7 +508,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     B[PH_NLEV] = n_lev;
     B[PH_NW] = nw;
     B[PH_IO] = io_off + j0;
-    B[PH_NSR] = nsr;
+    B[PH_NSR] = ports;
     B[PH_SRAM_OFF] = sram_off;
     B[PH_ISX] = isx != 0;
     B[PH_XOFF] = xoff;
@@ -683,8 +699,7 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
     stage_item[ms] = (uint32_t)(items.size() / 2);
     for (size_t b = 0; b < num_blocks; ++b) {
       const uint32_t c = entry[ms * num_blocks + b];
-      // an entry with an SRAM partition is not split
-      const uint32_t ks = (c >> 31) ? 1u : (uint32_t)nsub;
+      const uint32_t ks = (c >> 31) && !split_srams ? 1u : (uint32_t)nsub;
       for (uint32_t k = 0; k < (c & 0x7fffffffu); ++k, ++pid)
         for (uint32_t s = 0; s < ks; ++s) {
           items.push_back((uint32_t)pid);
@@ -733,6 +748,10 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
   blob = ws + lay.blob;
   item_off = B.item_off;
   item_words = B.item_words;
+  if ((r.unsupported & 4u) && split_srams) {  // once more without splitting those
+    split_srams = false;
+    return build(mode, want, round, pair_gates, ok);
+  }
   *ok = !r.unsupported;
   if (*ok && round) {
     std::vector<uint32_t> words(n_items), w2(n_items);

