@@ -6,9 +6,9 @@
 //
 // What bounds it: latency.  A major stage of one stream is a chain of state
 // word exchange, a few gate levels and the commit; an item's blob (up to
-// about 60 KB) is copied by TMA one item ahead.  us per pass, script form
-// before / plan: 16k gates x 64 cycles 2722 / 600, 2M gates x 16 cycles
-// 6130 / 1327, 256k gates x 16 cycles with checks 3466 / 1100.
+// about 60 KB) is copied by TMA one item ahead.  us per pass, script form / plan:
+// 16k gates x 64 cycles 2722 / 537, 2M gates x 16 cycles 6130 / 1224, 256k
+// gates x 32 cycles 4918 / 1486.
 #pragma once
 #include "plan_build.cuh"
 
@@ -188,7 +188,7 @@ __device__ __forceinline__ void plan_levels(const uint32_t *B, uint8_t *slots, u
   }
 }
 // PAIRS: every item of the plan is listed by pairs, so the kernel has one loop
-// (small design 555 us a pass with both, 537 with one).
+// (16k gates, 64 cycles: 555 us a pass with both, 537 with one).
 template <bool X, bool PAIRS>
 __device__ __forceinline__ void plan_gates(const uint32_t *B, uint8_t *slots, uint32_t ngr) {
   if (PAIRS || B[PH_PAIR])

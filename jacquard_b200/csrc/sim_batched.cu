@@ -1,5 +1,7 @@
 // Bit-lane batched interpreter for sm_100a: many independent stimulus streams
-// run the same script in one launch.
+// run the same script in one launch.  Scripts with a gate-list plan run
+// batched_plan.cuh; the kernels here run the prepared script (no plan, or
+// callers of jq_simulate_batched).
 //
 // Layout: a lane word is one u32 holding one signal of 32 streams, where
 // `signal` is the bit position of the plain layout (word*32 + bit) and the X

@@ -1,4 +1,9 @@
-// Plain interpreter kernel for sm_100a: the reference's script semantics
+// Plain interpreter for sm_100a, one stimulus stream.  Scripts with a gate-list
+// plan run plain_plan.cuh (host side below); this kernel runs the script form
+// itself: scripts without a plan, arrivals' tables, timed legacy calls, bounded
+// barrier waits.
+//
+// Script-form kernel: the reference's script semantics
 // (csrc/kernel_v1_impl.cuh:32-626), one stimulus stream, persistent over all
 // cycles of a launch with a bounded-wait grid barrier between major stages.
 //
@@ -500,9 +505,9 @@ constexpr uint32_t PLAN_GRID_ITEMS = 148;
 // The mirrored form's cluster (the largest, non-portable) and the snapshot it
 // may keep in shared memory.  It needs no L2 round trip between stages but
 // splits a stage into 16 items at most, so it serves stages of one or two
-// partitions: small 16k-gate design (1 partition, 16 items) 2.36 us a stage
-// against 2.85 in the flow form; 256k-gate SoC (3 partitions) 2.6 against 2.5
-// with 48 items.
+// partitions: small 16k-gate design (1 partition, 16 items) 2.10 us a stage
+// against 2.66 in the flow form; 256k-gate SoC (3 partitions, gates by level)
+// 2.6 against 2.5 with 48 items.
 constexpr uint32_t PLAN_CLUSTER = 16;
 constexpr size_t PLAN_MIRROR_PARTS = 2;
 constexpr size_t PLAN_MIRROR_BYTES = 112 * 1024;
