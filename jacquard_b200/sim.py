@@ -5,6 +5,7 @@ Device buffers are torch tensors (int32 storage for u32 words); every kernel
 call goes through libjacquard_b200.so -- there is no other execution path.
 """
 import ctypes
+import threading
 
 import numpy as np
 import torch
@@ -96,12 +97,18 @@ class DeviceScript:
         self._plan = None
         self._arrivals = None
         self._exchange = {}
+        # the tables below are made once, also when threads share the script
+        self._lock = threading.RLock()
 
     def plan(self, target_items=0):
         """The script's gate-list plan (jq_plain_plan_build), or None when the
         script is not one it represents; built on first use.  target_items is
         jq_plain_plan_build's (0: its default, PLAN_NO_MIRROR: never the form
         that keeps the state in shared memory)."""
+        with self._lock:
+            return self._make_plan(target_items)
+
+    def _make_plan(self, target_items):
         if self._plan is None:
             L = lib()
             dev = self.blocks_data.device
@@ -134,19 +141,24 @@ class DeviceScript:
             return None
         if stream is None:
             stream = torch.cuda.current_stream(self.blocks_data.device)
-        buf = self._exchange.get(stream.cuda_stream)
-        if buf is None:
-            with torch.cuda.stream(stream):
-                buf = torch.empty(n, dtype=torch.int32, device=self.blocks_data.device)
-            self._exchange[stream.cuda_stream] = buf
-        return buf.data_ptr()
+        with self._lock:
+            buf = self._exchange.get(stream.cuda_stream)
+            if buf is None:
+                with torch.cuda.stream(stream):
+                    buf = torch.empty(n, dtype=torch.int32, device=self.blocks_data.device)
+                self._exchange[stream.cuda_stream] = buf
+            return buf.data_ptr()
 
     def arrivals(self):
         """(first cycle's, later cycles') u16 arrival of every state word, in
         int32 device tensors; computed on first use."""
-        if self._arrivals is None:
-            self._arrivals = arrival_tables(self)
-        return self._arrivals
+        with self._lock:
+            if self._arrivals is None:
+                tables = arrival_tables(self)
+                # complete before a launch on any stream reads them
+                torch.cuda.current_stream(self.blocks_data.device).synchronize()
+                self._arrivals = tables
+            return self._arrivals
 
     def depth(self, stream=None):
         """(stage depth codes, per-entry base) on the device

@@ -173,3 +173,35 @@ def test_legacy_symbol_around_the_plan_rule(cycles):
     assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
     assert np.array_equal(sim.dev_to_u32(sram)[:wsram.size], wsram)
     assert np.array_equal(sim.dev_to_u32(sram_x)[:wsx.size], wsx)
+
+
+def test_first_timed_launch_on_another_stream_and_two_threads():
+    """The plan and the arrival tables are made inside the first launch; it may
+    be on another stream than the current one, and two threads may share the
+    script."""
+    import threading
+    s = cases.script("sram", 16, (8,), timing_seed=9)
+    s.enable_timing_arrivals()
+    try:
+        states = cases.stimulus("sram", s, 12)
+        cons = cases.constraint_buffer("sram", s, clock_ps=120, setup=30, hold=150)
+        off = s.arrival_state_offset
+        want, _, _, _ = run_oracle(s, states, 12, constraints=cons, cap=1 << 16, arrival_off=off)
+        ds = sim.DeviceScript(s)
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        outs = [None, None]
+
+        def work(k):
+            outs[k] = run(ds, s, states, 12, cons, 1 << 16, off, stream=streams[k])
+
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for k in range(2):
+            assert sim.status(streams[k]) == 0
+            assert np.array_equal(sim.dev_to_u32(outs[k][0]).reshape(states.shape), want)
+    finally:
+        s.timing_arrivals_enabled = False
+        s.arrival_state_offset = 0
