@@ -42,7 +42,8 @@ struct BPlanParams {
   const unsigned long long *item_off;
   const uint32_t *item_words;
   uint32_t stage_item[33];
-  uint32_t blob_cap, nbuf, slots;  // shared memory layout
+  // shared memory layout (slots: a multiple of 16 bytes)
+  uint32_t blob_cap, nbuf, slots;
 };
 
 // The part of a slot one thread handles: (value, X) words of its lane words,

@@ -2706,13 +2706,16 @@ int jq_batched_plan_build(const size_t *blocks_start, const uint32_t *blocks_dat
   // item's slots do not fit
   const uint32_t pair_gates = bplan_pair_gates(lanes_per_item, x);
   bool pairs = true;
+  // slots of an item as a multiple of 16 bytes (what follows them in shared
+  // memory is read in 8-byte words)
+  const uint32_t slot_words = lanes_per_item * (x ? 2u : 1u), unit = slot_words < 4 ? 4 / slot_words : 1;
   for (size_t want = round;;) {
     rc = b.build(PLAN_SIGNALS, want, round, plan->paired ? 0xffffffffu : 0u, &ok);
     if (rc != JQ_OK) return rc;
     plan->supported = 0;
     if (ok) {
       plan->max_blob = b.r.max_blob;
-      plan->max_slots = b.r.max_slots;
+      plan->max_slots = (b.r.max_slots + unit - 1) / unit * unit;
       plan->nbuf = bplan_smem(plan, 2) <= lim ? 2 : bplan_smem(plan, 1) <= lim ? 1 : 0;
       plan->widest = b.widest;
       for (size_t ms = 0; ms <= 32; ++ms) plan->stage_item[ms] = b.stage_item[ms];
