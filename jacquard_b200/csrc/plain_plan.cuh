@@ -306,7 +306,6 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
   uint32_t *const buf0 = reinterpret_cast<uint32_t *>(dyn);
   uint8_t *const slots = dyn + 4 * (size_t)P.nbuf * P.blob_cap;
   uint2 *const words = reinterpret_cast<uint2 *>(slots + P.slot_bytes);
-  uint2 *const old0 = words + P.gw_cap;  // [2][256]
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t rank = blockIdx.x, G = gridDim.x, nms = P.num_major_stages;
   if (t == 0) {
@@ -328,7 +327,6 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
       const uint32_t i1 = P.stage_item[ms + 1];
       for (uint32_t it = P.stage_item[ms] + rank; it < i1; it += G) {
         const uint32_t *B = buf0 + (size_t)F.buf_of(n_run) * P.blob_cap;
-        uint2 *const old = old0 + 256 * (n_run & 1u);
         // the blob of this item (copied while the last one ran)
         bool ok = plan_mbar_wait(&bar[F.buf_of(n_run)], F.par_of(n_run));
         if (!opened && t == 0 && c >= 3) {
@@ -367,8 +365,11 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
         const uint32_t ngw = B[PH_NGW], ngr = B[PH_NGR], nw = B[PH_NW];
         const uint32_t io = B[PH_IO];
         const bool isx = X && B[PH_ISX] != 0;
-        // ---- state words, and the old words of writeouts that may keep them
-        // (this CTA wrote those)
+        // ---- state words, and the old words of writeouts that may keep them:
+        // lane k of warp w commits writeout word w + 16 k of the item in every
+        // cycle, so it reads what it wrote itself, in its own program order
+        const uint32_t my_j = warp + (EB / 32) * lane;
+        uint2 old = make_uint2(0, 0);
         if (ok) {
           const uint32_t *gw = B + B[PH_OGW];
           constexpr int K = 4;  // words in flight per thread
@@ -423,9 +424,8 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
             for (int k = 0; k < K; ++k)
               if (i0 + k * EB < ngw) words[i0 + k * EB] = make_uint2(v[k], x[k]);
           }
-          const uint32_t j = EB - 1 - t;
-          if (j < nw && B[B[PH_OKEEP] + j])
-            old[j] = make_uint2(ldcg(in + io + j), isx ? ldcg(in + (size_t)P.xoff + io + j) : 0u);
+          if (my_j < nw && B[B[PH_OKEEP] + my_j])
+            old = make_uint2(ldcg(in + io + my_j), isx ? ldcg(in + (size_t)P.xoff + io + my_j) : 0u);
         }
         // a wait that ran out ends the launch with its status set
         if (__syncthreads_or(!ok)) {
@@ -451,18 +451,17 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
         plan_srams(P, B, slots, isx);
         // ---- commit: a warp per writeout word
         {
-          const uint32_t *com = B + B[PH_OCOM], *kp = B + B[PH_OKEEP];
+          const uint32_t *com = B + B[PH_OCOM];
           for (uint32_t j = warp; j < nw; j += EB / 32) {
             const PlanWord w = plan_word(com, slots, j, isx);
-            if (lane == 0) {
-              const uint2 ow = kp[j] ? old[j] : make_uint2(0, 0);
+            if (my_j == j) {
               const size_t o = (size_t)io + j;
               const size_t at = (size_t)((c + 1) & 3) * P.rio + o;
               const uint32_t n = (uint32_t)(c + 1);
-              const uint32_t nv = (ow.x & ~w.cp) | (w.v & w.cp);
+              const uint32_t nv = (old.x & ~w.cp) | (w.v & w.cp);
               if (X) {
                 // a partition without X leaves the snapshot's host-filled X word
-                const uint32_t nx = isx ? (ow.y & ~w.cp & ~w.cx) | (w.x & w.cp & ~w.cx) | w.cx
+                const uint32_t nx = isx ? (old.y & ~w.cp & ~w.cx) | (w.x & w.cp & ~w.cx) | w.cx
                                         : ldcg(out + P.xoff + o);
                 asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(
                                  reinterpret_cast<uint4 *>(P.exchange) + at),

@@ -520,11 +520,11 @@ constexpr uint32_t PLAN_PAIR_GATES = 400;
 constexpr uint32_t PLAN_GRID_ONLY = 0xffffffffu;  // target_items: never the mirrored form
 
 // Shared memory of the executor: blob buffers and slots, then the state
-// words and old words of an item, or the two mirrored snapshots.
+// words of an item, or the two mirrored snapshots.
 size_t plan_smem_bytes(const jq_plain_plan *p, uint32_t nbuf) {
   const size_t base = 4 * (size_t)nbuf * p->max_blob + ((p->max_slots + 15) & ~15u);
   return base + (p->mirrored ? 2 * (size_t)p->rio * (p->xoff ? 8 : 4)
-                             : 8 * (size_t)((p->max_gw + 1) & ~1u) + 2 * 8 * 256);
+                             : 8 * (size_t)((p->max_gw + 1) & ~1u));
 }
 
 template <bool X, bool PAIRS>
