@@ -49,7 +49,8 @@ struct PlanParams {
   int slot;
 };
 
-static __device__ unsigned long long g_plan_count[BAR_SLOTS], g_plan_hint[BAR_SLOTS];
+// g_plan_count[slot][k]: arrivals of cycles c with c mod 4 = k (see plan_flow_kernel)
+static __device__ unsigned long long g_plan_count[BAR_SLOTS][4], g_plan_hint[BAR_SLOTS];
 
 // plan_mbar_wait for words other CTAs of the cluster sent.
 __device__ __forceinline__ bool plan_mbar_wait_cluster(uint64_t *bar, uint32_t parity) {
@@ -290,7 +291,11 @@ __device__ __forceinline__ uint2 plan_poll(const uint2 *p) {
 // published in buffer k mod 4 with the number k (zeroed before the launch;
 // words that no partition writes are read from the snapshot itself).  The
 // buffer of snapshot c + 1 held snapshot c - 3, so a CTA starts cycle c when
-// every CTA is done with the loads of cycle c - 3.
+// every CTA is done with the loads of cycle c - 3.  Each CTA arrives once per
+// cycle, in the counter of the cycle mod 4: nothing holds a CTA back from one
+// that only reads its words, so one sum over all cycles would let the CTAs
+// ahead stand in for one behind, and its words would be overwritten.  No CTA
+// arrives for cycle c + 4 before every CTA has arrived for c.
 //
 // Hint.  With many CTAs the polls of those that wait slow down the words the
 // others publish, so above PLAN_HINT_ITEMS items a stage a CTA first waits
@@ -330,13 +335,13 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
         // the blob of this item (copied while the last one ran)
         bool ok = plan_mbar_wait(&bar[F.buf_of(n_run)], F.par_of(n_run));
         if (!opened && t == 0 && c >= 3) {
-          const unsigned long long target = (unsigned long long)P.active * (c - 2);
+          const unsigned long long target = (unsigned long long)P.active * ((c - 3) / 4 + 1);
           const uint64_t t0 = clock64();
           for (;;) {
             unsigned long long v;
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
                          : "=l"(v)
-                         : "l"(&g_plan_count[P.slot])
+                         : "l"(&g_plan_count[P.slot][(c - 3) & 3])
                          : "memory");
             if (v >= target) break;
             if (*((volatile int *)&g_status[P.slot]) != 0 ||
@@ -434,7 +439,8 @@ __global__ void __launch_bounds__(EB, 1) plan_flow_kernel(const __grid_constant_
           return;
         }
         if (!opened && t == 0 && c)  // done with the loads of cycle c - 1
-          asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&g_plan_count[P.slot])
+          asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(
+                           &g_plan_count[P.slot][(c - 1) & 3])
                        : "memory");
         opened = true;
         if (two && t == PT) F.issue();  // into the other buffer: its readers passed this barrier

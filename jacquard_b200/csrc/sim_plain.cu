@@ -438,7 +438,7 @@ namespace {
 // it is captured in CUDA graphs together with the launch).
 __global__ void jq_plain_reset_kernel(int slot) {
   g_bar_count[slot] = 0;
-  g_plan_count[slot] = 0;
+  for (int k = 0; k < 4; ++k) g_plan_count[slot][k] = 0;
   g_plan_hint[slot] = 0;
   g_status[slot] = 0;
 }

@@ -1,10 +1,13 @@
 """Planned runs (one-stream and batched) where their memory layout, the order
 of their CTAs or their choice of form can go wrong, against the CPU oracle."""
+import numpy as np
 import pytest
+import torch
 
 import cases
 import test_gpu_batched as tgb
-from jacquard_b200 import batched
+from jacquard_b200 import batched, frontend, sim, state
+from test_gpu_plain import run_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -18,3 +21,58 @@ def test_timed_single_lane_items_without_x_of_any_slot_count():
         assert plan is not None and plan.lanes_per_item == 1
         assert plan.max_slots % 4 == 0  # before any launch
         tgb.test_batched_setup_hold_events_match_oracle_per_stream(False, lanes, per_item, parts)
+
+
+def one_way_design(n_src=512, n_sink=512, depth=64, seed=5):
+    """Registers that only depend on themselves (shift and XOR), and registers
+    that nothing reads behind `depth` levels of gates over them."""
+    lib = frontend._lib()
+    rng = np.random.default_rng(seed)
+    b = lib.jqf_builder_new()
+    clk = lib.jqf_builder_clock_flag(b)
+    x = lib.jqf_builder_input(b) << 1
+    q = [lib.jqf_builder_dff(b) << 1 for _ in range(n_src + n_sink)]
+
+    def and_(u, v):
+        return lib.jqf_builder_and(b, u, v)
+
+    for i in range(n_src):
+        u, v = q[i - 1] if i else x, q[(i * 7 + 3) % n_src]
+        assert lib.jqf_builder_set_dff(b, i, and_(and_(u, v) ^ 1, and_(u ^ 1, v ^ 1) ^ 1), clk << 1) == 0
+    for k in range(n_sink):
+        s = q[k % n_src]
+        for _ in range(depth):
+            s = and_(s ^ int(rng.integers(2)), q[int(rng.integers(n_src))] ^ int(rng.integers(2))) ^ 1
+        assert lib.jqf_builder_set_dff(b, n_src + k, s, clk << 1) == 0
+    lib.jqf_builder_output(b, q[n_src])
+    assert lib.jqf_builder_finish(b, clk, 0) == 0
+    return frontend.Design.from_handle(b), n_src
+
+
+@pytest.mark.parametrize("xprop", [False, True])
+@pytest.mark.parametrize("parts", [3, 6])
+def test_producers_do_not_run_ahead_of_consumers(parts, xprop):
+    """One-way dependencies in the flow form: nothing but the ring's own count
+    holds the CTAs of the sources back from those of the much slower sinks,
+    whose words they overwrite four cycles later."""
+    d, n_src = one_way_design()
+    s = d.build_script(num_blocks=16, xprop=xprop, target_parts=parts, merge_passes=0)
+    assert s.num_major_stages == 1
+    word = state.dff_positions(s, d) >> 5
+    src, sink = set(word[:n_src].tolist()), set(word[n_src:].tolist())
+    assert len(src - sink) >= 8  # words (and so items) of sources alone
+    cycles = 400
+    states = state.random_stimulus_states(s, d, cycles, 3)
+    if xprop:
+        states = state.expand_states_for_xprop(states, s)
+    states[0, :s.reg_io_state_size] |= np.random.default_rng(1).integers(
+        0, 2**32, s.reg_io_state_size, dtype=np.uint32)
+    want, _, _, _ = run_oracle(s, states, cycles)
+    ds = sim.DeviceScript(s)
+    assert not ds.plan(sim.PLAN_NO_MIRROR).mirrored
+    for _ in range(3):
+        st = sim.u32_to_dev(states.reshape(-1))
+        z = torch.zeros(1, dtype=torch.int32, device="cuda")
+        sim.simulate(ds, st, cycles, states.shape[1], z, z)
+        assert sim.status() == 0
+        assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
