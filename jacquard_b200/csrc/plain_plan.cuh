@@ -685,7 +685,14 @@ __global__ void __launch_bounds__(EB, 1) plan_mirror_kernel(const __grid_constan
   if (failed && t == 0) atomicCAS(&g_status[P.slot], 0, JQ_ERR_BARRIER_TIMEOUT);
   if (t == PT) F.drain(n_run);
   // no CTA leaves while another may still send it words (on failure the
-  // others' bounded waits end too)
+  // others' bounded waits end too), nor before the last stage's words have
+  // arrived: the barrier below orders the sends, not their arrival
+  if (t == 0 && !failed && P.num_cycles && rank < P.active) {
+    const size_t lc = P.num_cycles - 1;
+    if (!plan_mbar_wait_cluster(&stage_bar[2 * (nms - 1) + (uint32_t)(lc & 1)],
+                                (uint32_t)(lc >> 1) & 1u))
+      atomicCAS(&g_status[P.slot], 0, JQ_ERR_BARRIER_TIMEOUT);
+  }
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }

@@ -76,3 +76,22 @@ def test_producers_do_not_run_ahead_of_consumers(parts, xprop):
         sim.simulate(ds, st, cycles, states.shape[1], z, z)
         assert sim.status() == 0
         assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
+
+
+@pytest.mark.parametrize("cycles", [1, 2, 3, 5])
+def test_short_mirrored_launches_in_a_row(cycles):
+    """The cluster form's CTAs end only when the words sent to them have
+    arrived: many short launches, each on the state the last one left."""
+    s = cases.script("small", 64, (8, 16, 24))
+    ds = sim.DeviceScript(s)
+    assert ds.plan().mirrored
+    n = 40 * cycles
+    states = cases.stimulus("small", s, n)
+    want, _, _, _ = run_oracle(s, states, n)
+    st = sim.u32_to_dev(states.reshape(-1))
+    z = torch.zeros(1, dtype=torch.int32, device="cuda")
+    eff = states.shape[1]
+    for k in range(0, n, cycles):
+        sim.simulate(ds, st[k * eff:], cycles, eff, z, z)
+    assert sim.status() == 0
+    assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
