@@ -636,6 +636,12 @@ size_t plan_smem_limit(const void *fn) {
   return (size_t)optin - fa.sharedSizeBytes;
 }
 
+bool plan_smem_allow(const void *fn) {
+  const size_t lim = plan_smem_limit(fn);
+  return lim && cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lim) ==
+                    cudaSuccess;
+}
+
 const uint32_t *PlanBuilder::unwritten() const {
   return ws + PlanLayout(num_blocks * nms, parts, 0, state_words).unwritten;
 }

@@ -97,6 +97,10 @@ size_t plan_workspace_words(size_t blocks_data_len, size_t num_blocks, size_t nm
 
 // Opt-in shared memory per CTA left for the dynamic part of fn.
 size_t plan_smem_limit(const void *fn);
+// Lets fn have all of it.  The attribute is the function's, not the launch's:
+// set to what one plan needs, a launch of a larger plan by another thread
+// would be refused.
+bool plan_smem_allow(const void *fn);
 
 // mbarrier wait with a bound of about a second.
 __device__ __forceinline__ uint32_t plan_smem(const void *p) {

@@ -2447,9 +2447,8 @@ int jq_batched_smem_bytes(uint32_t wo_slots) {
 
 static int variant_max_blocks(int device, uint32_t wo_slots, Variant v, size_t *max_blocks) {
   const void *fn = variant_fn(v);
-  const int smem = (int)smem_layout_bytes(wo_slots, v);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return JQ_ERR_LAUNCH;
+  const size_t smem = smem_layout_bytes(wo_slots, v);
+  if (smem > plan_smem_limit(fn) || !plan_smem_allow(fn)) return JQ_ERR_LAUNCH;
   int sms = 0, per = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, BT, smem) != cudaSuccess)
@@ -2768,8 +2767,7 @@ int jq_simulate_batched_planned(const jq_batch_args *a, const jq_batched_plan *p
   cudaStream_t st = (cudaStream_t)a->stream;
   const void *fn = bplan_fn(p, P.constraints != nullptr);
   const int smem = (int)bplan_smem(p, p->nbuf);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-    return JQ_ERR_LAUNCH;
+  if (!plan_smem_allow(fn)) return JQ_ERR_LAUNCH;
   jq_batched_reset_kernel<<<1, 1, 0, st>>>(P.slot);
   if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
   void *args[] = {&P, &Q};

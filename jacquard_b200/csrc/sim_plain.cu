@@ -553,8 +553,7 @@ int plan_cluster_launch(const jq_plain_plan *p, PlanParams *P, cudaStream_t st, 
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)cfg.dynamicSmemBytes) != cudaSuccess ||
+  if (!plan_smem_allow(fn) ||
       cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return JQ_ERR_LAUNCH;
   if (query) {
@@ -669,7 +668,7 @@ int launch_planned(const jq_sim_args *a, const jq_plain_plan *p, const uint32_t 
   if (p->mirrored) return plan_cluster_launch(p, &P, st, false);
   const int smem = (int)plan_smem_bytes(p, p->nbuf);
   const void *fn = plan_fn(p);
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+  if (!plan_smem_allow(fn) ||
       cudaMemsetAsync(exchange, 0, p->exchange_words * 4, st) != cudaSuccess)
     return JQ_ERR_LAUNCH;
   void *args[] = {&P};

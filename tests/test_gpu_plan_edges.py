@@ -1,5 +1,7 @@
 """Planned runs (one-stream and batched) where their memory layout, the order
 of their CTAs or their choice of form can go wrong, against the CPU oracle."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -95,3 +97,64 @@ def test_short_mirrored_launches_in_a_row(cycles):
         sim.simulate(ds, st[k * eff:], cycles, eff, z, z)
     assert sim.status() == 0
     assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
+
+
+def _threads(*works):
+    errors = []
+
+    def guard(w):
+        try:
+            w()
+        except Exception as e:  # reported by the caller's assertion
+            errors.append(e)
+
+    ts = [threading.Thread(target=guard, args=(w,)) for w in works]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+
+
+def test_two_threads_launch_plans_of_different_size():
+    """Two threads launch the same kernel for scripts whose plans need very
+    different shared memory, each on its own stream; then the same for
+    batched runs.  No launch is refused."""
+    scripts = [cases.script("tiny", 8, (5,), xprop=True),
+               cases.script("soc_mini", 148, (20, 40, 60), xprop=True, target_parts=37)]
+    kinds, works, check = ("tiny", "soc_mini"), [], []
+    dss = [sim.DeviceScript(s) for s in scripts]
+    plans = [ds.plan(sim.PLAN_NO_MIRROR) for ds in dss]
+    assert plans[0].paired == plans[1].paired and plans[1].max_slots > 2 * plans[0].max_slots
+    for k, s, ds in zip(kinds, scripts, dss):
+        states = cases.stimulus(k, s, 2, x_init=True)
+        st = sim.u32_to_dev(states.reshape(-1))
+        n = max(1, s.sram_storage_size)
+        sram, sram_x = (torch.zeros(n, dtype=torch.int32, device="cuda") for _ in range(2))
+        q = torch.cuda.Stream()
+
+        def work(ds=ds, st=st, eff=states.shape[1], sram=sram, sram_x=sram_x, q=q):
+            for _ in range(400):
+                sim.simulate(ds, st, 2, eff, sram, sram_x, stream=q)
+
+        works.append(work)
+        check.append(q)
+    torch.cuda.synchronize()
+    _threads(*works)
+    for q in check:
+        assert sim.status(q) == 0
+    works = []
+    sims = [batched.BatchedSim(s, 2, lanes_per_item=2) for s in scripts]
+    assert sims[0].plan.paired == sims[1].plan.paired
+    for B in sims:
+        B.load_state(np.zeros((2, B.sig), np.uint32))
+        q = torch.cuda.Stream()
+
+        def work(B=B, q=q):
+            for _ in range(400):
+                B.run(None, 2, stream=q)
+            assert B.status(q) == 0
+
+        works.append(work)
+    torch.cuda.synchronize()
+    _threads(*works)
