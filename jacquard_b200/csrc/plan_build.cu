@@ -13,7 +13,7 @@ struct PlanBuildParams {
   const uint32_t *part_ms;             // its major stage
   const uint32_t *items;               // per item: partition, sub | nsub << 16
   const uint32_t *writer;              // per state word: major stage + 1 that writes it, or 0
-  uint32_t writer_words;
+  uint32_t read_end;                   // words below it are values (X words lie above)
   uint32_t mode;                       // PlanMode
   uint32_t pair_gates;                 // gates a level up to which levels go in pairs
   uint32_t *blob;
@@ -107,8 +107,8 @@ __device__ __forceinline__ bool plan_and(uint32_t a, uint32_t b, uint32_t xa, ui
 // represent -- a writeout slot that no hook, SRAM or duplicate writes, or a
 // permutation that reads one an earlier partition left (both observe the
 // per-block arrays of the script kernel), a partition that reads what the
-// same major stage writes, or sizes past the limits above -- and the script
-// then runs in its own form.
+// same major stage writes or X words as values, or sizes past the limits
+// above -- and the script then runs in its own form.
 __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, uint32_t n_items) {
   extern __shared__ __align__(16) uint8_t plan_dyn[];
   PlanShared &ps = *reinterpret_cast<PlanShared *>(plan_dyn);
@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
       const uint32_t w = im.x & 0x7fffffffu;
       // staged reads: only words that earlier major stages (or nobody) write
       if (hit && (im.x >> 31)) {
-        if (w < P.writer_words && P.writer[w] > my_ms) bad = true;
+        if (w < P.read_end && P.writer[w] > my_ms) bad = true;
       }
-      if (hit && w >= P.writer_words) bad = true;
+      if (hit && w >= P.read_end) bad = true;
     }
   }
   uint32_t n_gw = 0, n_gr = 0;
@@ -527,11 +527,12 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
 
 // Partition offsets and major stages of every entry, and the major stage
 // that writes each state word (writer, zeroed; two writers of one word make
-// the plan unsupported: their order within a block matters).
+// the plan unsupported: their order within a block matters).  srams: (first
+// word, SRAMs) of the partitions with SRAMs, any order.
 __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *script,
                                  const uint32_t *part_base, unsigned entries, unsigned num_blocks,
                                  unsigned long long *part_off, uint32_t *part_ms, uint32_t *writer,
-                                 uint32_t writer_words, PlanResult *res) {
+                                 uint32_t writer_words, uint2 *srams, PlanResult *res) {
   const unsigned e = blockIdx.x;
   if (e >= entries) return;
   size_t off = blocks_start[e];
@@ -547,6 +548,8 @@ __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *scr
       atomicMax(&res->rio, io + nio);
       atomicAdd(&res->stage_words[ms], nio);
       atomicOr(&res->x_use, script[off + 8] ? 2u : 1u);
+      if (script[off + 4])
+        srams[atomicAdd(&res->n_sram_parts, 1u)] = make_uint2(script[off + 5], script[off + 4]);
       if (script[off + 8]) {
         atomicMax(&res->xoff_max, script[off + 9]);
         atomicMax(&res->xoff_inv_max, ~script[off + 9]);
@@ -562,9 +565,22 @@ __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *scr
   }
 }
 
-// The words below res->rio that no partition writes (inputs), any order.
+// The words below res->rio that no partition writes (inputs), any order; and
+// the plan unsupported when two partitions share an SRAM (their order within
+// a block, or their major stages, decide what they read).
 __global__ void plan_unwritten_kernel(const uint32_t *writer, uint32_t writer_words,
-                                      uint32_t *list, uint32_t cap, PlanResult *res) {
+                                      uint32_t *list, uint32_t cap, const uint2 *srams,
+                                      PlanResult *res) {
+  const uint32_t n = res->n_sram_parts;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const uint2 a = srams[i];
+    const unsigned long long a1 = a.x + (unsigned long long)a.y * SRAM_WORDS;
+    for (uint32_t j = 0; j < i; ++j) {
+      const uint2 b = srams[j];
+      if (b.x < a1 && a.x < b.x + (unsigned long long)b.y * SRAM_WORDS)
+        atomicOr(&res->unsupported, 1u);
+    }
+  }
   for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < res->rio && w < writer_words;
        w += gridDim.x * blockDim.x)
     if (!writer[w]) {
@@ -594,7 +610,7 @@ namespace {
 
 // Layout of the plan build's workspace (words; the blobs take the rest).
 struct PlanLayout {
-  size_t part_base, part_ms, part_off, writer, unwritten, items, item_words, item_off, blob;
+  size_t part_base, part_ms, part_off, srams, writer, unwritten, items, item_words, item_off, blob;
   PlanLayout(size_t entries, size_t parts, size_t n_items, size_t writer_words) {
     size_t w = (sizeof(PlanResult) / 4 + 3) & ~(size_t)3;
     auto take = [&](size_t n) {
@@ -605,6 +621,7 @@ struct PlanLayout {
     part_base = take(entries);
     part_ms = take(parts);
     part_off = take(2 * parts);
+    srams = take(2 * parts);
     writer = take(writer_words);
     unwritten = take(writer_words);
     items = take(2 * n_items);
@@ -680,15 +697,17 @@ int PlanBuilder::scan(bool *ok) {
   plan_list_kernel<<<(unsigned)entries, 64, 0, st>>>(
       blocks_start, blocks_data, ws + l1.part_base, (unsigned)entries, (unsigned)num_blocks,
       reinterpret_cast<unsigned long long *>(ws + l1.part_off), ws + l1.part_ms, ws + l1.writer,
-      (uint32_t)state_words, res);
+      (uint32_t)state_words, reinterpret_cast<uint2 *>(ws + l1.srams), res);
   plan_unwritten_kernel<<<64, 256, 0, st>>>(ws + l1.writer, (uint32_t)state_words,
-                                            ws + l1.unwritten, (uint32_t)state_words, res);
+                                            ws + l1.unwritten, (uint32_t)state_words,
+                                            reinterpret_cast<const uint2 *>(ws + l1.srams), res);
   if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
   if (cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return JQ_ERR_CUDA;
-  // one X offset for every partition with X
-  const bool one_xoff = !(r.x_use & 2u) || (r.xoff_max == ~r.xoff_inv_max && r.xoff_max > 0);
+  // one X offset for every partition with X, above the value words
+  const bool one_xoff =
+      !(r.x_use & 2u) || (r.xoff_max == ~r.xoff_inv_max && r.xoff_max > 0 && r.rio <= r.xoff_max);
   *ok = !r.unsupported && one_xoff;
   return JQ_OK;
 }
@@ -733,7 +752,8 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
   B.part_ms = ws + lay.part_ms;
   B.items = ws + lay.items;
   B.writer = ws + lay.writer;
-  B.writer_words = (uint32_t)state_words;
+  B.read_end = (uint32_t)state_words;
+  if ((r.x_use & 2u) && r.xoff_max < state_words) B.read_end = r.xoff_max;
   B.mode = mode;
   B.pair_gates = pair_gates;
   B.blob = ws + lay.blob;

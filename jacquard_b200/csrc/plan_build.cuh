@@ -55,7 +55,8 @@ struct PlanResult {
   uint32_t max_blob, max_slots, max_gw, rio;
   uint32_t xoff_max, xoff_inv_max, n_unwritten;
   uint32_t max_level;     // most gates per level of any item, on average
-  uint32_t unpaired, pad;  // an item lists its gates by level
+  uint32_t unpaired;  // an item lists its gates by level
+  uint32_t n_sram_parts;  // partitions with SRAMs
   uint32_t stage_words[32];
 };
 

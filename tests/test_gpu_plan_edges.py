@@ -9,7 +9,7 @@ import torch
 import cases
 import test_gpu_batched as tgb
 from jacquard_b200 import batched, frontend, sim, state
-from test_gpu_plain import run_oracle
+from test_gpu_plain import run_gpu, run_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -158,3 +158,67 @@ def test_two_threads_launch_plans_of_different_size():
         works.append(work)
     torch.cuda.synchronize()
     _threads(*works)
+
+
+class Edited:
+    """A script with its own copy of the instruction words."""
+
+    def __init__(self, s):
+        self.__dict__.update(s.__dict__)
+        self.blocks_data = s.blocks_data.copy()
+
+    def partitions(self):
+        """(major stage, block, word offset) in script order."""
+        bd, out = self.blocks_data, []
+        for e in range(self.num_major_stages * self.num_blocks):
+            off = int(self.blocks_start[e])
+            while bd[off]:
+                out.append((e // self.num_blocks, e % self.num_blocks, off))
+                if bd[off + 1]:
+                    break
+                off += 256 + 512 * int(bd[off + 6]) + 5120 * (int(bd[off]) + 2)
+        return out
+
+
+def script_form(b, states, cycles):
+    """(snapshots, SRAM, SRAM X) of a run of the script's own form."""
+    st = sim.u32_to_dev(states.reshape(-1))
+    n = max(1, b.sram_storage_size)
+    sram = torch.zeros(n, dtype=torch.int32, device="cuda")
+    sram_x = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    sim.simulate(sim.DeviceScript(b), st, cycles, states.shape[1], sram, sram_x, planned=False)
+    assert sim.status() == 0
+    return sim.dev_to_u32(st).reshape(states.shape), sim.dev_to_u32(sram), sim.dev_to_u32(sram_x)
+
+
+def check_without_plan(b, states, cycles, want):
+    """No plan of either kind, and every entry point gives the script's result."""
+    assert sim.DeviceScript(b).plan() is None
+    for legacy in (False, True):
+        got = run_gpu(b, states, cycles, legacy=legacy)[:3]
+        for g, w in zip(got, want):
+            assert np.array_equal(g[:w.size] if g.ndim == 1 else g, w)
+    assert batched.BatchedSim(b, 2).plan is None
+
+
+def test_shared_sram_and_x_words_read_as_values_have_no_plan():
+    """Two partitions of a block on one SRAM run in the block's order, and a
+    read of another partition's X word as a value needs the barrier of its
+    major stage: the plan orders neither, so the script runs in its own form."""
+    s = cases.script("sram", 1, (), xprop=True, target_parts=4)
+    states = cases.stimulus("sram", s, 40, x_init=True)
+    b = Edited(s)
+    ports = [off for _, _, off in b.partitions() if b.blocks_data[off + 4]]
+    assert len(ports) == 3
+    b.blocks_data[ports[1] + 5] = b.blocks_data[ports[0] + 5]
+    check_without_plan(b, states, 40, run_oracle(b, states, 40)[:3])
+
+    s = cases.script("sram", 16, (8,), xprop=True, target_parts=4)
+    states = cases.stimulus("sram", s, 40, x_init=True)
+    b = Edited(s)
+    bd = b.blocks_data
+    first, second = [[o for m, _, o in b.partitions() if m == k] for k in (0, 1)]
+    g = bd[first[0] + 256:first[0] + 256 + 512].reshape(-1, 2)
+    k = int(np.nonzero(g[:, 1])[0][0])
+    g[k, 0] = bd[second[0] + 9] + bd[second[0] + 3] + 1  # an X word stage 1 writes
+    check_without_plan(b, states, 40, script_form(b, states, 40))
