@@ -94,49 +94,58 @@ class DeviceScript:
             np.ascontiguousarray(script.blocks_start, dtype=np.uint64).view(np.int64)).to(device)
         self.blocks_data = u32_to_dev(script.blocks_data, device)
         self._depth = None
-        self._plan = None
+        self._plan = None  # the plan in use: (plan, its workspace)
+        self._plans = {}   # by target_items
         self._arrivals = None
         self._exchange = {}
         # the tables below are made once, also when threads share the script
         self._lock = threading.RLock()
 
     def plan(self, target_items=0):
-        """The script's gate-list plan (jq_plain_plan_build), or None when the
-        script is not one it represents; built on first use.  target_items is
-        jq_plain_plan_build's (0: its default, PLAN_NO_MIRROR: never the form
-        that keeps the state in shared memory)."""
+        """The script's gate-list plan (jq_plain_plan_build) that simulate()
+        runs from then on, or None when the script is not one it represents;
+        built on first use.  target_items is jq_plain_plan_build's (0: its
+        default, PLAN_NO_MIRROR: never the form that keeps the state in shared
+        memory); simulate() alone uses the default."""
         with self._lock:
-            return self._make_plan(target_items)
+            if target_items not in self._plans:
+                self._plans[target_items] = self._make_plan(target_items)
+            self._plan = self._plans[target_items]
+            return self._plan[0]
+
+    def plan_in_use(self):
+        """The plan simulate() runs: the last one asked for, else the default."""
+        with self._lock:
+            return self.plan() if self._plan is None else self._plan[0]
 
     def _make_plan(self, target_items):
-        if self._plan is None:
-            L = lib()
-            dev = self.blocks_data.device
-            rio = self.script.reg_io_state_size
-            n = L.jq_plain_plan_words(self.blocks_data.numel(), self.num_blocks,
-                                      self.num_major_stages, rio)
-            ws = torch.empty(n, dtype=torch.int32, device=dev)
-            p = PlainPlan()
-            rc = L.jq_plain_plan_build(self.blocks_start.data_ptr(), self.blocks_data.data_ptr(),
-                                       self.num_blocks, self.num_major_stages, rio, target_items,
-                                       ws.data_ptr(), n, ctypes.byref(p), torch.cuda.current_stream(dev).cuda_stream)
-            if rc:
-                raise RuntimeError("jq_plain_plan_build: " + L.jq_strerror(rc).decode())
-            if p.supported:  # keep the used part only
-                used = ws[:p.used_words].clone()
-                for f in ("blob", "item_off", "item_words", "unwritten"):
-                    setattr(p, f, getattr(p, f) - ws.data_ptr() + used.data_ptr())
-                torch.cuda.current_stream(dev).synchronize()
-                self._plan = (p, used)
-            else:
-                self._plan = (None, None)
-        return self._plan[0]
+        """(plan or None, its workspace)"""
+        L = lib()
+        dev = self.blocks_data.device
+        rio = self.script.reg_io_state_size
+        n = L.jq_plain_plan_words(self.blocks_data.numel(), self.num_blocks,
+                                  self.num_major_stages, rio)
+        ws = torch.empty(n, dtype=torch.int32, device=dev)
+        p = PlainPlan()
+        rc = L.jq_plain_plan_build(self.blocks_start.data_ptr(), self.blocks_data.data_ptr(),
+                                   self.num_blocks, self.num_major_stages, rio, target_items,
+                                   ws.data_ptr(), n, ctypes.byref(p), torch.cuda.current_stream(dev).cuda_stream)
+        if rc:
+            raise RuntimeError("jq_plain_plan_build: " + L.jq_strerror(rc).decode())
+        if p.supported:  # keep the used part only
+            used = ws[:p.used_words].clone()
+            for f in ("blob", "item_off", "item_words", "unwritten"):
+                setattr(p, f, getattr(p, f) - ws.data_ptr() + used.data_ptr())
+            torch.cuda.current_stream(dev).synchronize()
+            return p, used
+        return None, None
 
-    def exchange(self, stream=None):
-        """Device pointer of the exchange buffer for planned launches on this
-        stream (one per stream, allocated on it, so launches on two streams
-        may overlap; kept with the script), or None when the plan needs none."""
-        n = self._plan[0].exchange_words
+    def exchange(self, stream=None, plan=None):
+        """Device pointer of the exchange buffer for launches of `plan` (the
+        one in use) on this stream (one per stream, allocated on it, so launches
+        on two streams may overlap; kept with the script, as large for each of
+        its plans that needs one), or None when the plan needs none."""
+        n = (plan or self.plan_in_use()).exchange_words
         if not n:
             return None
         if stream is None:
@@ -219,13 +228,13 @@ def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=
         # the plan and the arrival tables are made on first use, which a
         # stream capture cannot record: such a call runs the script's own form
         ready = ds._plan is not None and (ds._arrivals is not None or not tracked)
-        plan = ds.plan() if ready or not _capturing(stream) else None
+        plan = ds.plan_in_use() if ready or not _capturing(stream) else None
         if plan is not None:
             first = steady = None
             if tracked:
                 first, steady = (t.data_ptr() for t in ds.arrivals())
             rc = lib().jq_simulate_planned(ctypes.byref(a), ctypes.byref(plan), first, steady,
-                                           ds.exchange(stream))
+                                           ds.exchange(stream, plan))
             if rc:
                 raise RuntimeError("jq_simulate: " + lib().jq_strerror(rc).decode())
             return

@@ -222,3 +222,29 @@ def test_shared_sram_and_x_words_read_as_values_have_no_plan():
     k = int(np.nonzero(g[:, 1])[0][0])
     g[k, 0] = bd[second[0] + 9] + bd[second[0] + 3] + 1  # an X word stage 1 writes
     check_without_plan(b, states, 40, script_form(b, states, 40))
+
+
+def test_each_asked_for_plan_is_its_own():
+    """plan(target) gives the plan of that target whatever was built before,
+    and simulate() runs the one asked for last."""
+    s = cases.script("small", 64, (8, 16, 24))
+    states = cases.stimulus("small", s, 20)
+    want, _, _, _ = run_oracle(s, states, 20)
+    ds = sim.DeviceScript(s)
+    z = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def run():
+        st = sim.u32_to_dev(states.reshape(-1))
+        sim.simulate(ds, st, 20, states.shape[1], z, z)
+        assert sim.status() == 0
+        assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
+
+    run()
+    first = ds.plan()
+    assert first.mirrored
+    for target, items in [(sim.PLAN_NO_MIRROR, None), (5, 5), (0, 16)]:
+        plan = ds.plan(target)
+        assert bool(plan.mirrored) == (target != sim.PLAN_NO_MIRROR)
+        assert items is None or plan.widest == items
+        run()
+    assert ds.plan() is first
