@@ -309,7 +309,10 @@ class BatchedSim:
             return False
         n = L.jq_batched_plan_words(self.ds.blocks_data.numel(), self.ds.num_blocks,
                                     self.ds.num_major_stages, rio)
-        ws = torch.empty(n, dtype=torch.int32, device=self.device)
+        try:
+            ws = torch.empty(n, dtype=torch.int32, device=self.device)
+        except torch.cuda.OutOfMemoryError:  # the prepared script takes less
+            return False
         p = BatchedPlan()
         rc = L.jq_batched_plan_build(self.ds.blocks_start.data_ptr(), self.ds.blocks_data.data_ptr(),
                                      self.ds.num_blocks, self.ds.num_major_stages, rio, self.lanes,
@@ -319,7 +322,10 @@ class BatchedSim:
             raise RuntimeError("jq_batched_plan_build: " + sim.lib().jq_strerror(rc).decode())
         if not p.supported or p.num_partitions != self.num_partitions:
             return False
-        used = ws[:p.used_words].clone()  # the used part only
+        try:
+            used = ws[:p.used_words].clone()  # the used part only
+        except torch.cuda.OutOfMemoryError:
+            return False
         for f in ("blob", "item_off", "item_words"):
             setattr(p, f, getattr(p, f) - ws.data_ptr() + used.data_ptr())
         torch.cuda.current_stream(self.device).synchronize()

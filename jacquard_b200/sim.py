@@ -103,13 +103,19 @@ class DeviceScript:
 
     def plan(self, target_items=0):
         """The script's gate-list plan (jq_plain_plan_build) that simulate()
-        runs from then on, or None when the script is not one it represents;
-        built on first use.  target_items is jq_plain_plan_build's (0: its
-        default, PLAN_NO_MIRROR: never the form that keeps the state in shared
-        memory); simulate() alone uses the default."""
+        runs from then on, or None when the script is not one it represents
+        or its workspace cannot be allocated; built on first use.
+        target_items is jq_plain_plan_build's (0: its default, PLAN_NO_MIRROR:
+        never the form that keeps the state in shared memory); simulate()
+        alone uses the default."""
         with self._lock:
             if target_items not in self._plans:
-                self._plans[target_items] = self._make_plan(target_items)
+                try:
+                    self._plans[target_items] = self._make_plan(target_items)
+                except torch.cuda.OutOfMemoryError:
+                    # the script's own form runs in less; plan() tries again
+                    self._plan = (None, None)
+                    return None
             self._plan = self._plans[target_items]
             return self._plan[0]
 
@@ -211,11 +217,16 @@ def _capturing(stream):
 def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=None,
              events=None, event_capacity=0, arrival_state_offset=0, first_cycle=0,
              stream=None, barrier_timeout_cycles=0, skip_dead_levels=True, planned=True):
-    """Launch the plain interpreter (asynchronous).  All tensors on device.
+    """Launch the plain interpreter (asynchronous, but for the first call on a
+    script: it builds the script's plan in a workspace larger than the script,
+    or its stage-depth tables, and waits for them; a first call with arrivals
+    or constraints also runs two cycles for the arrival tables).  All tensors
+    on device.
     skip_dead_levels: pass the script's stage-depth tables, so tree levels
     whose outputs nothing reads are skipped (False runs every level).
-    planned: run the script's gate-list plan when it has one and the barrier
-    wait is not bounded by the caller (skip_dead_levels only)."""
+    planned: run the script's gate-list plan when it has one, the memory for it
+    is there and the barrier wait is not bounded by the caller
+    (skip_dead_levels only)."""
     a = SimArgs(ds.num_blocks, ds.num_major_stages, ds.blocks_start.data_ptr(),
                 ds.blocks_data.data_ptr(), sram.data_ptr(),
                 sram_x.data_ptr() if sram_x is not None else None, num_cycles, state_size,
@@ -231,10 +242,14 @@ def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=
         plan = ds.plan_in_use() if ready or not _capturing(stream) else None
         if plan is not None:
             first = steady = None
-            if tracked:
-                first, steady = (t.data_ptr() for t in ds.arrivals())
-            rc = lib().jq_simulate_planned(ctypes.byref(a), ctypes.byref(plan), first, steady,
-                                           ds.exchange(stream, plan))
+            try:
+                if tracked:
+                    first, steady = (t.data_ptr() for t in ds.arrivals())
+                buf = ds.exchange(stream, plan)
+            except torch.cuda.OutOfMemoryError:
+                plan = None
+        if plan is not None:
+            rc = lib().jq_simulate_planned(ctypes.byref(a), ctypes.byref(plan), first, steady, buf)
             if rc:
                 raise RuntimeError("jq_simulate: " + lib().jq_strerror(rc).decode())
             return

@@ -248,3 +248,34 @@ def test_each_asked_for_plan_is_its_own():
         assert items is None or plan.widest == items
         run()
     assert ds.plan() is first
+
+
+def test_no_memory_for_a_plan(monkeypatch):
+    """A plan's workspace that cannot be allocated: the script's own form (one
+    stream) and the prepared script (batched) run, and a later plan() builds it."""
+    huge = 1 << 42  # words
+    monkeypatch.setattr(sim.lib(), "jq_plain_plan_words", lambda *a: huge)
+    monkeypatch.setattr(batched.lib(), "jq_batched_plan_words", lambda *a: huge)
+    s = cases.script("sram", 16, (8,), xprop=True)
+    states = cases.stimulus("sram", s, 10, x_init=True)
+    want, _, _, _ = run_oracle(s, states, 10)
+    ds = sim.DeviceScript(s)
+
+    def run():
+        st = sim.u32_to_dev(states.reshape(-1))
+        n = s.sram_storage_size
+        sim.simulate(ds, st, 10, states.shape[1], torch.zeros(n, dtype=torch.int32, device="cuda"),
+                     torch.full((n,), -1, dtype=torch.int32, device="cuda"))
+        assert sim.status() == 0
+        assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
+
+    run()
+    assert ds.plan() is None
+    c = tgb.BatchedCase("sram", s, 2)
+    assert c.B.plan is None
+    c.launch()
+    assert c.B.status() == 0
+    c.verify()
+    monkeypatch.undo()
+    assert ds.plan() is not None
+    run()
