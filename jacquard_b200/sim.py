@@ -128,7 +128,9 @@ class DeviceScript:
         """(plan or None, its workspace)"""
         L = lib()
         dev = self.blocks_data.device
-        rio = self.script.reg_io_state_size
+        rio = getattr(self.script, "reg_io_state_size", None)
+        if rio is None:  # launch arrays alone (the layout is the caller's)
+            return None, None
         n = L.jq_plain_plan_words(self.blocks_data.numel(), self.num_blocks,
                                   self.num_major_stages, rio)
         ws = torch.empty(n, dtype=torch.int32, device=dev)
@@ -159,7 +161,7 @@ class DeviceScript:
         with self._lock:
             buf = self._exchange.get(stream.cuda_stream)
             if buf is None:
-                with torch.cuda.stream(stream):
+                with torch.cuda.stream(_torch_stream(stream, self.blocks_data.device)):
                     buf = torch.empty(n, dtype=torch.int32, device=self.blocks_data.device)
                 self._exchange[stream.cuda_stream] = buf
             return buf.data_ptr()
@@ -207,10 +209,19 @@ def max_blocks(device=0):
     return n.value
 
 
-def _capturing(stream):
+def _torch_stream(stream, device):
+    """`stream` as a torch stream; any object with a cuda_stream handle does."""
+    if isinstance(stream, torch.cuda.Stream):
+        return stream
+    if not stream.cuda_stream:
+        return torch.cuda.default_stream(device)
+    return torch.cuda.ExternalStream(stream.cuda_stream, device=device)
+
+
+def _capturing(stream, device):
     if stream is None:
         return torch.cuda.is_current_stream_capturing()
-    with torch.cuda.stream(stream):
+    with torch.cuda.stream(_torch_stream(stream, device)):
         return torch.cuda.is_current_stream_capturing()
 
 
@@ -239,7 +250,7 @@ def simulate(ds, states, num_cycles, state_size, sram, sram_x=None, constraints=
         # the plan and the arrival tables are made on first use, which a
         # stream capture cannot record: such a call runs the script's own form
         ready = ds._plan is not None and (ds._arrivals is not None or not tracked)
-        plan = ds.plan_in_use() if ready or not _capturing(stream) else None
+        plan = ds.plan_in_use() if ready or not _capturing(stream, ds.blocks_data.device) else None
         if plan is not None:
             first = steady = None
             try:

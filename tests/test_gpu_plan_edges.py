@@ -279,3 +279,33 @@ def test_no_memory_for_a_plan(monkeypatch):
     monkeypatch.undo()
     assert ds.plan() is not None
     run()
+
+
+def test_plain_stream_handles_and_bare_launch_arrays():
+    """simulate() takes any object with a cuda_stream handle as the stream, and
+    a DeviceScript of nothing but the launch arrays."""
+    class Handle:
+        def __init__(self, stream):
+            self.cuda_stream = stream.cuda_stream
+
+    class Arrays:
+        def __init__(self, s):
+            for f in ("num_blocks", "num_major_stages", "blocks_start", "blocks_data"):
+                setattr(self, f, getattr(s, f))
+
+    s = cases.script("sram", 16, (8,), timing_seed=9)
+    n = s.sram_storage_size
+    for script, off in [(s, 0), (Arrays(s), 0), (Arrays(s), s.reg_io_state_size)]:
+        states = cases.stimulus("sram", s, 10)
+        if off:
+            states = state.expand_states_for_arrivals(states, s)
+        want, _, _, _ = run_oracle(s, states, 10, arrival_off=off)
+        q = torch.cuda.Stream()
+        for handle in (q, Handle(q), Handle(torch.cuda.default_stream())):
+            st = sim.u32_to_dev(states.reshape(-1))
+            sram = torch.zeros(n, dtype=torch.int32, device="cuda")
+            torch.cuda.synchronize()
+            sim.simulate(sim.DeviceScript(script), st, 10, states.shape[1], sram, sram,
+                         arrival_state_offset=off, stream=handle)
+            assert sim.status(handle) == 0
+            assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
