@@ -790,9 +790,9 @@ struct PlanCache {
   size_t words = 0;
 };
 PlanCache g_plan_cache[64];
-// One legacy call at a time per process: they share the workspaces above, and
-// each waits for its launch anyway.
-std::mutex g_legacy_mutex;
+// One legacy call at a time per device: they share its workspaces above, and
+// each waits for its launch anyway.  (Index 64: devices without workspaces.)
+std::mutex g_legacy_mutex[65];
 
 // Runs an untimed legacy call on a plan built for it; false when the script
 // has none or the workspace cannot be had, and then the script's own form
@@ -847,7 +847,9 @@ bool legacy_planned(const jq_sim_args *a, int *rc) {
 void legacy_launch(const jq_sim_args *a0, uint32_t event_cap, const char *what) {
   jq_sim_args a1 = *a0;
   jq_sim_args *a = &a1;
-  std::lock_guard<std::mutex> lock(g_legacy_mutex);
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 64) dev = 64;
+  std::lock_guard<std::mutex> lock(g_legacy_mutex[dev]);
   int rc = JQ_OK;
   if (!legacy_planned(a, &rc)) {
     legacy_depth(a);

@@ -309,3 +309,19 @@ def test_plain_stream_handles_and_bare_launch_arrays():
                          arrival_state_offset=off, stream=handle)
             assert sim.status(handle) == 0
             assert np.array_equal(sim.dev_to_u32(st).reshape(states.shape), want)
+
+
+def test_two_threads_call_the_reference_symbol():
+    """Calls on one device take turns and keep to their own scripts."""
+    works = []
+    for kind, nb, split in (("tiny", 8, (5,)), ("sram", 16, (8,))):
+        s = cases.script(kind, nb, split)
+        states = cases.stimulus(kind, s, 20)
+        want, _, _, _ = run_oracle(s, states, 20)
+
+        def work(s=s, states=states, want=want):
+            for _ in range(10):
+                assert np.array_equal(run_gpu(s, states, 20, legacy=True)[0], want)
+
+        works.append(work)
+    _threads(*works)
