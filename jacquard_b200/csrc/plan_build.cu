@@ -10,7 +10,6 @@ constexpr int PB = 1024;  // threads of the build kernel
 struct PlanBuildParams {
   const uint32_t *script;
   const unsigned long long *part_off;  // script word offset of each partition
-  const uint32_t *part_ms;             // its major stage
   const uint32_t *items;               // per item: partition, sub | nsub << 16
   const uint32_t *writer;              // per state word: major stage + 1 that writes it, or 0
   uint32_t read_end;                   // words below it are values (X words lie above)
@@ -104,11 +103,10 @@ __device__ __forceinline__ bool plan_and(uint32_t a, uint32_t b, uint32_t xa, ui
 // last item has the ports, the duplicate and the SRAM slots, the others share
 // the hooked slots (flag bit 2 when one of them reads an SRAM's output).  The
 // result's `unsupported` flag is set for what the plan does not
-// represent -- a writeout slot that no hook, SRAM or duplicate writes, or a
-// permutation that reads one an earlier partition left (both observe the
-// per-block arrays of the script kernel), a partition that reads what the
-// same major stage writes or X words as values, or sizes past the limits
-// above -- and the script then runs in its own form.
+// represent -- a permutation that reads a writeout slot an earlier partition
+// left (the per-block arrays of the script kernel), X words read as values, or
+// sizes past the limits above; the kernels below find the rest -- and the
+// script then runs in its own form.
 __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, uint32_t n_items) {
   extern __shared__ __align__(16) uint8_t plan_dyn[];
   PlanShared &ps = *reinterpret_cast<PlanShared *>(plan_dyn);
@@ -119,13 +117,12 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
   const uint32_t *m = P.script + P.part_off[pid];
   const uint32_t ns = m[0], nio = m[2], io_off = m[3], nsr = m[4], sram_off = m[5], R = m[6],
                  ndup = m[7], isx = m[8], xoff = m[9];
-  const uint32_t my_ms = P.part_ms[pid];
-  bool bad = ns > PLAN_MAX_NS || nio > 256 || nsr * 4 + ndup > 256 || nsr + ndup > nio ||
-             R > 32;
-  if (bad) {  // uniform
-    if (t == 0) atomicOr(&P.res->unsupported, 1u);
-    return;
-  }
+  bool bad = false;
+  // another item found the script to be one without a plan
+  auto given_up = [&]() {
+    return __syncthreads_or(t == 0 && (*(volatile uint32_t *)&P.res->unsupported & 1u));
+  };
+  if (given_up()) return;
   const uint32_t *gr = m + 256, *ch = gr + 512 * (size_t)R;
   const uint32_t hooked = nio - nsr - ndup;  // slots below are hooked
   uint32_t j0 = nio * sub / nsub, j1 = nio * (sub + 1) / nsub;
@@ -173,11 +170,6 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
       if ((p >> 5) >= hooked) bad = true;  // (reads no SRAM or duplicate slot: wneed of
       else atomicOr(&ps.wneed[p >> 5], 1u << (p & 31));  // those is complete)
     }
-  }
-  __syncthreads();
-  for (uint32_t j = t; j < hooked; j += PB) {
-    const uint32_t hw = m[128 + j / 2], h = (j & 1) ? hw >> 16 : hw & 0xffffu;
-    if (ps.wneed[j] && (h >> 8) >= ns) bad = true;
   }
   if (__syncthreads_or(bad)) {
     if (t == 0) atomicOr(&P.res->unsupported, 1u);
@@ -251,10 +243,6 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
       n_ent += hit != 0;
       n_bit += hit;
       const uint32_t w = im.x & 0x7fffffffu;
-      // staged reads: only words that earlier major stages (or nobody) write
-      if (hit && (im.x >> 31)) {
-        if (w < P.read_end && P.writer[w] > my_ms) bad = true;
-      }
       if (hit && w >= P.read_end) bad = true;
     }
   }
@@ -272,6 +260,11 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     }
     __syncthreads();
   };
+  if (__syncthreads_or(bad)) {
+    if (t == 0) atomicOr(&P.res->unsupported, 1u);
+    return;
+  }
+  if (given_up()) return;
   // ---- forward over the stages: reference of every live position; with
   // `gates` the gates are written, else counted per level
   auto forward = [&](uint32_t *gates, uint32_t gate0, bool pair) {
@@ -527,7 +520,9 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
 
 // Partition offsets and major stages of every entry, and the major stage
 // that writes each state word (writer, zeroed; two writers of one word make
-// the plan unsupported: their order within a block matters).  srams: (first
+// the plan unsupported: their order within a block matters; so do partitions
+// past the limits of the build and writeout slots without a hook, here, so
+// that the build is spared).  srams: (first
 // word, SRAMs) of the partitions with SRAMs, any order.
 __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *script,
                                  const uint32_t *part_base, unsigned entries, unsigned num_blocks,
@@ -541,7 +536,16 @@ __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *scr
   for (;;) {
     const uint32_t ns = script[off];
     if (!ns) break;
-    const uint32_t nio = script[off + 2], io = script[off + 3];
+    const uint32_t nio = script[off + 2], io = script[off + 3], nsr = script[off + 4],
+                   ndup = script[off + 7];
+    bool bad = ns > PLAN_MAX_NS || nio > 256 || nsr * 4 + ndup > 256 || nsr + ndup > nio ||
+               script[off + 6] > 32;
+    if (!bad)
+      for (uint32_t j = threadIdx.x; j < nio - nsr - ndup; j += blockDim.x) {
+        const uint32_t hw = script[off + 128 + j / 2], h = (j & 1) ? hw >> 16 : hw & 0xffffu;
+        bad |= (h >> 8) >= ns;
+      }
+    if (bad) atomicOr(&res->unsupported, 1u);
     if (threadIdx.x == 0) {
       part_off[pid] = off;
       part_ms[pid] = ms;
@@ -567,10 +571,23 @@ __global__ void plan_list_kernel(const size_t *blocks_start, const uint32_t *scr
 
 // The words below res->rio that no partition writes (inputs), any order; and
 // the plan unsupported when two partitions share an SRAM (their order within
-// a block, or their major stages, decide what they read).
+// a block, or their major stages, decide what they read) or a partition reads
+// what its own major stage writes.
 __global__ void plan_unwritten_kernel(const uint32_t *writer, uint32_t writer_words,
                                       uint32_t *list, uint32_t cap, const uint2 *srams,
-                                      PlanResult *res) {
+                                      const uint32_t *script, const unsigned long long *part_off,
+                                      const uint32_t *part_ms, uint32_t parts, PlanResult *res) {
+  for (uint32_t pid = blockIdx.x; pid < parts; pid += gridDim.x) {
+    const uint32_t *m = script + part_off[pid];
+    const uint32_t ms = part_ms[pid], entries = 256 * m[6];
+    bool bad = false;
+    for (uint32_t i = threadIdx.x; i < entries; i += blockDim.x) {
+      const uint2 im = ldg2(m + 256 + 2 * i);
+      const uint32_t w = im.x & 0x7fffffffu;
+      bad |= im.y && (im.x >> 31) && w < writer_words && writer[w] > ms;
+    }
+    if (bad) atomicOr(&res->unsupported, 1u);
+  }
   const uint32_t n = res->n_sram_parts;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint2 a = srams[i];
@@ -698,9 +715,11 @@ int PlanBuilder::scan(bool *ok) {
       blocks_start, blocks_data, ws + l1.part_base, (unsigned)entries, (unsigned)num_blocks,
       reinterpret_cast<unsigned long long *>(ws + l1.part_off), ws + l1.part_ms, ws + l1.writer,
       (uint32_t)state_words, reinterpret_cast<uint2 *>(ws + l1.srams), res);
-  plan_unwritten_kernel<<<64, 256, 0, st>>>(ws + l1.writer, (uint32_t)state_words,
-                                            ws + l1.unwritten, (uint32_t)state_words,
-                                            reinterpret_cast<const uint2 *>(ws + l1.srams), res);
+  plan_unwritten_kernel<<<256, 256, 0, st>>>(
+      ws + l1.writer, (uint32_t)state_words, ws + l1.unwritten, (uint32_t)state_words,
+      reinterpret_cast<const uint2 *>(ws + l1.srams), blocks_data,
+      reinterpret_cast<const unsigned long long *>(ws + l1.part_off), ws + l1.part_ms,
+      (uint32_t)parts, res);
   if (cudaGetLastError() != cudaSuccess) return JQ_ERR_LAUNCH;
   if (cudaMemcpyAsync(&r, res, sizeof r, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
@@ -749,7 +768,6 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
   PlanBuildParams B;
   B.script = blocks_data;
   B.part_off = reinterpret_cast<unsigned long long *>(ws + lay.part_off);
-  B.part_ms = ws + lay.part_ms;
   B.items = ws + lay.items;
   B.writer = ws + lay.writer;
   B.read_end = (uint32_t)state_words;

@@ -325,3 +325,36 @@ def test_two_threads_call_the_reference_symbol():
 
         works.append(work)
     _threads(*works)
+
+
+def spoiled(spoil):
+    """A script that has no plan, whose result the order of its blocks decides."""
+    s = cases.script("tiny", 1, (5,), target_parts=4)
+    b = Edited(s)
+    bd = b.blocks_data
+    offs = [o for m, _, o in b.partitions() if m == 0]
+    last = offs[-1]
+    if spoil == "stale slot":
+        bd[last + 128] |= 0xFFFF  # slot 0 without a hook
+    elif spoil == "same stage":
+        g = bd[last + 256:last + 256 + 512].reshape(-1, 2)
+        k = int(np.nonzero(g[:, 1])[0][0])
+        g[k, 0] = 0x80000000 | int(bd[offs[0] + 3])  # the first partition's word, staged
+    else:
+        bd[last + 3] = bd[offs[0] + 3]
+    return s, b
+
+
+@pytest.mark.parametrize("spoil", ["stale slot", "same stage", "two writers"])
+def test_refused_scripts_give_the_oracles_result(spoil):
+    """Scripts that the plan does not represent, each spoiled in its last
+    partition, in one block (so that the result is defined): one-stream runs,
+    the script form and the reference symbol give the oracle's snapshots."""
+    s, b = spoiled(spoil)
+    states = cases.stimulus("tiny", s, 20)
+    want = run_oracle(b, states, 20)[0]
+    assert sim.DeviceScript(b).plan() is None
+    assert batched.BatchedSim(b, 2).plan is None
+    assert np.array_equal(run_gpu(b, states, 20)[0], want)
+    assert np.array_equal(script_form(b, states, 20)[0], want)
+    assert np.array_equal(run_gpu(b, states, 20, legacy=True)[0], want)
