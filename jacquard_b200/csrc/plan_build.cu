@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(PB, 1) plan_build_kernel(PlanBuildParams P, ui
     ps.off = atomicAdd(&P.res->used, (unsigned long long)words);
     if (ps.off + words > P.blob_cap) {
       ps.bad = 1;
-      atomicOr(&P.res->unsupported, 1u);
+      atomicOr(&P.res->unsupported, 8u);
     } else {
       P.item_off[item] = ps.off;
       P.item_words[item] = words;
@@ -660,6 +660,12 @@ size_t plan_workspace_words(size_t blocks_data_len, size_t num_blocks, size_t nm
          blocks_data_len + nms * PLAN_SPARE_ITEMS * 1024 + 4096;
 }
 
+size_t plan_workspace_first(size_t blocks_data_len, size_t num_blocks, size_t nms,
+                            size_t state_words) {
+  const size_t all = plan_workspace_words(blocks_data_len, num_blocks, nms, state_words);
+  return all - blocks_data_len / 2;
+}
+
 size_t plan_smem_limit(const void *fn) {
   int dev = 0, optin = 0;
   cudaFuncAttributes fa;
@@ -797,6 +803,7 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
     return build(mode, want, round, pair_gates, ok);
   }
   *ok = !r.unsupported;
+  overflow = r.unsupported == 8u;
   if (*ok && round) {
     std::vector<uint32_t> words(n_items), w2(n_items);
     std::vector<unsigned long long> off(n_items), o2(n_items);

@@ -44,7 +44,7 @@ enum PlanHdr : uint32_t {
 };
 
 // Build result: unsupported flag (bit 0: the plan, bit 1: its mirrored form, bit
-// 2: splitting partitions with SRAMs),
+// 2: splitting partitions with SRAMs, bit 3: the workspace was too small),
 // blob words used, the largest blob, slot count and state-word count of any
 // item, the words up to the last written one, X use (bit 0: a partition
 // without, bit 1: with X) and its offset (min and ~max), the words each major
@@ -77,7 +77,8 @@ struct PlanBuilder {
   // of the last build()
   uint32_t stage_item[33];
   uint32_t widest;
-  size_t used_words;
+  size_t used_words;  // (what it takes, when `overflow`)
+  bool overflow = false;  // only the workspace's size stood in its way
   const uint32_t *blob, *item_words;
   const unsigned long long *item_off;
 
@@ -94,6 +95,10 @@ struct PlanBuilder {
 
 // Words of workspace a build of any script of this size fits in.
 size_t plan_workspace_words(size_t blocks_data_len, size_t num_blocks, size_t nms,
+                            size_t state_words);
+
+// The same with item blobs of at most half of the script.
+size_t plan_workspace_first(size_t blocks_data_len, size_t num_blocks, size_t nms,
                             size_t state_words);
 
 // Opt-in shared memory per CTA left for the dynamic part of fn.

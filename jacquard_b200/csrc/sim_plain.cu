@@ -568,9 +568,11 @@ int plan_cluster_launch(const jq_plain_plan *p, PlanParams *P, cudaStream_t st, 
   return cudaLaunchKernelExC(&cfg, fn, args) == cudaSuccess ? JQ_OK : JQ_ERR_LAUNCH;
 }
 
+// With `need`, a build that only lacks workspace ends there and says how many
+// words it takes.
 int plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t num_blocks,
                size_t nms, size_t state_words, uint32_t target, uint32_t *ws, size_t ws_words,
-               jq_plain_plan *plan, cudaStream_t st) {
+               jq_plain_plan *plan, cudaStream_t st, size_t *need = nullptr) {
   *plan = jq_plain_plan{};
   plan->num_blocks = num_blocks;
   plan->num_major_stages = nms;
@@ -591,6 +593,10 @@ int plan_build(const size_t *blocks_start, const uint32_t *blocks_data, size_t n
                                                            : PLAN_GRID_ITEMS;
     rc = b.build(mirrored ? PLAN_MIRROR : PLAN_WORDS, want, 0, PLAN_PAIR_GATES, &ok);
     if (rc != JQ_OK) return rc;
+    if (need && b.overflow) {
+      *need = b.used_words;
+      return JQ_OK;
+    }
     if (ok) {
       plan->mirrored = mirrored;
       plan->paired = !b.r.unpaired;
@@ -780,8 +786,11 @@ int read_status(void *stream) {
 }
 
 // Plan workspace of the legacy wrappers, per device: kept up to this many
-// bytes, given back after the call above.
-constexpr size_t LEGACY_PLAN_KEEP = 256u << 20;
+// bytes, given back after the call above.  A script of up to twice this size
+// first tries this much: a plan takes a fourteenth (2M gates, 148 flat
+// partitions a stage) to a half of its script, and allocating and freeing
+// 900 MB in every call took 1.3 ms of a 256k-gate script's (872 MB, plan 262).
+constexpr size_t LEGACY_PLAN_KEEP = 512u << 20;
 // Cycles from which a legacy call builds the plan: the build takes 0.2 ms for
 // a 16k-gate and 1.4 ms for a 2M-gate design and saves 34 us and 300 us a cycle.
 constexpr size_t LEGACY_PLAN_CYCLES = 8;
@@ -808,24 +817,36 @@ bool legacy_planned(const jq_sim_args *a, int *rc) {
   if (cudaMemcpy(&len, a->blocks_start + a->num_blocks * a->num_major_stages, sizeof len,
                  cudaMemcpyDeviceToHost) != cudaSuccess)
     return false;
-  const size_t plan_words = (jq_plain_plan_words(len, a->num_blocks, a->num_major_stages,
-                                                 a->state_size) + 3) & ~(size_t)3;
-  const size_t words = plan_words + 16 * a->state_size;  // exchange buffer at the end
-  PlanCache &pc = g_plan_cache[dev];
-  if (pc.words < words) {
-    if (pc.ws) cudaFree(pc.ws);
-    pc = PlanCache{};
-    if (cudaMalloc(&pc.ws, words * 4) != cudaSuccess) {
-      cudaGetLastError();
-      pc.ws = nullptr;
-      return false;
-    }
-    pc.words = words;
+  // (an exchange buffer of 16 words a state word lies behind the plan)
+  size_t plan_words = jq_plain_plan_words(len, a->num_blocks, a->num_major_stages, a->state_size);
+  if (4 * (plan_words + 16 * a->state_size) > LEGACY_PLAN_KEEP) {
+    const size_t first =
+        plan_workspace_first(len, a->num_blocks, a->num_major_stages, a->state_size);
+    if (4 * (first + 16 * a->state_size) < LEGACY_PLAN_KEEP)
+      plan_words = LEGACY_PLAN_KEEP / 4 - 16 * a->state_size - 4;
   }
+  PlanCache &pc = g_plan_cache[dev];
   jq_plain_plan plan;
-  const bool ok = plan_build(a->blocks_start, a->blocks_data, a->num_blocks, a->num_major_stages,
-                             a->state_size, 0, pc.ws, plan_words, &plan, nullptr) == JQ_OK &&
-                  plan.supported;
+  bool ok = false;
+  for (size_t need = plan_words; need;) {
+    plan_words = (need + 3) & ~(size_t)3;
+    const size_t words = plan_words + 16 * a->state_size;
+    if (pc.words < words) {
+      if (pc.ws) cudaFree(pc.ws);
+      pc = PlanCache{};
+      if (cudaMalloc(&pc.ws, words * 4) != cudaSuccess) {
+        cudaGetLastError();
+        pc.ws = nullptr;
+        return false;
+      }
+      pc.words = words;
+    }
+    plan_words = pc.words - 16 * a->state_size;
+    need = 0;
+    ok = plan_build(a->blocks_start, a->blocks_data, a->num_blocks, a->num_major_stages,
+                    a->state_size, 0, pc.ws, plan_words, &plan, nullptr, &need) == JQ_OK &&
+         plan.supported;
+  }
   if (ok) {
     *rc = launch_planned(a, &plan, nullptr, nullptr, pc.ws + plan_words);
     if (*rc == JQ_OK) *rc = read_status(nullptr);
