@@ -139,8 +139,8 @@ int jq_sim_status(void *stream);
  * script order.  With stage_depth NULL only *num_stages (the size needed) is
  * computed.  JQ_ERR_INVALID_ARG when depth_capacity is too small.
  * Synchronizes `stream`.  The legacy wrappers build the script's gate-list plan
- * (below) for untimed calls of 8 cycles or more, and otherwise compute these
- * tables, into device buffers the library keeps per device (grown for larger
+ * (below) for untimed calls of 8 cycles or more (more for large scripts and few
+ * major stages), and otherwise compute these tables, into device buffers the library keeps per device (grown for larger
  * scripts; a plan workspace above 512 MB is given back after the call). */
 int jq_plain_prepare(const size_t *blocks_start, const uint32_t *blocks_data, size_t num_blocks,
                      size_t num_major_stages, uint32_t *stage_depth_base, uint8_t *stage_depth,

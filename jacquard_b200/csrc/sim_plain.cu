@@ -791,9 +791,13 @@ int read_status(void *stream) {
 // partitions a stage) to a half of its script, and allocating and freeing
 // 900 MB in every call took 1.3 ms of a 256k-gate script's (872 MB, plan 262).
 constexpr size_t LEGACY_PLAN_KEEP = 512u << 20;
-// Cycles from which a legacy call builds the plan: the build takes 0.2 ms for
-// a 16k-gate and 1.4 ms for a 2M-gate design and saves 34 us and 300 us a cycle.
-constexpr size_t LEGACY_PLAN_CYCLES = 8;
+// When a legacy call builds the plan: from 8 cycles on, and major stages times
+// cycles of at least 12 plus one per 8M script words.  The plan saves a stage's
+// latency in every cycle and its build grows with the script.  us a call,
+// script form / plan: 1,500 gates in one stage x 8 cycles 192 / 214, x 12
+// 228 / 220; in two stages x 8 236 / 210; 256k gates in four stages of 55M words
+// x 8 6,930 / 7,130, x 10 8,350 / 7,560; 256k gates in 20 stages x 8 1,330 / 845.
+constexpr size_t LEGACY_PLAN_CYCLES = 8, LEGACY_PLAN_STAGES = 12, LEGACY_PLAN_LEN = 8u << 20;
 struct PlanCache {
   uint32_t *ws = nullptr;
   size_t words = 0;
@@ -816,6 +820,9 @@ bool legacy_planned(const jq_sim_args *a, int *rc) {
   size_t len = 0;
   if (cudaMemcpy(&len, a->blocks_start + a->num_blocks * a->num_major_stages, sizeof len,
                  cudaMemcpyDeviceToHost) != cudaSuccess)
+    return false;
+  if (a->num_cycles < (LEGACY_PLAN_STAGES + len / LEGACY_PLAN_LEN + a->num_major_stages - 1) /
+                          a->num_major_stages)
     return false;
   // (an exchange buffer of 16 words a state word lies behind the plan)
   size_t plan_words = jq_plain_plan_words(len, a->num_blocks, a->num_major_stages, a->state_size);

@@ -358,3 +358,14 @@ def test_refused_scripts_give_the_oracles_result(spoil):
     assert np.array_equal(run_gpu(b, states, 20)[0], want)
     assert np.array_equal(script_form(b, states, 20)[0], want)
     assert np.array_equal(run_gpu(b, states, 20, legacy=True)[0], want)
+
+
+@pytest.mark.parametrize("kind,nb,split,cycles", [
+    ("tiny", 4, (), 8), ("tiny", 4, (), 11), ("tiny", 4, (), 12), ("tiny", 8, (5,), 7),
+    ("tiny", 8, (5,), 8)])
+def test_reference_symbol_around_the_stage_rule(kind, nb, split, cycles):
+    """The symbol builds the plan from 8 cycles and 12 stages on."""
+    s = cases.script(kind, nb, split)
+    states = cases.stimulus(kind, s, cycles)
+    want, _, _, _ = run_oracle(s, states, cycles)
+    assert np.array_equal(run_gpu(s, states, cycles, legacy=True)[0], want)
