@@ -247,6 +247,8 @@ class BatchedSim:
                 self.plan, self._plan_ws, self.x_interleaved = octets
         if self.plan is None:
             self._prepared()
+        else:  # (octet_need() may have made it; made again where it is read)
+            self._prep = None
         regions = getattr(script, "input_regions", None)
         if regions is None:
             self.in_sigs = input_words(script) * 32

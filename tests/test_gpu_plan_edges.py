@@ -369,3 +369,13 @@ def test_reference_symbol_around_the_stage_rule(kind, nb, split, cycles):
     states = cases.stimulus(kind, s, cycles)
     want, _, _, _ = run_oracle(s, states, cycles)
     assert np.array_equal(run_gpu(s, states, cycles, legacy=True)[0], want)
+
+
+def test_planned_octets_do_not_keep_the_prepared_script():
+    """Asking for octet items checks the prepared script's capacity; a run on
+    the plan does not read that script, and it is made again where it is."""
+    s = cases.script("sram", 16, (8,), xprop=True, target_parts=16)
+    B = batched.BatchedSim(s, 8, lanes_per_item=8)
+    assert B.plan is not None and B._prep is None
+    assert B.prepared.numel() == B.ds.blocks_data.numel()
+    assert B.octet_need() <= batched.octet_capacity()
