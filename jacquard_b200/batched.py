@@ -194,6 +194,9 @@ def check_x_offsets(script, value_words):
             off += 256 + 512 * int(bd[off + 6]) + 5120 * (ns + 2)
 
 
+PLAN_ITEM_PARTITION = 18  # word of an item's header (PH_PART in plan_build.cuh)
+
+
 class BatchedSim:
     """Script + buffers on the device for `lanes` lane words (32*lanes streams)."""
 
@@ -338,6 +341,17 @@ class BatchedSim:
         """Words of the plan's item blobs: what a cycle streams of the script."""
         lo = (self.plan.item_words - self._plan_ws.data_ptr()) // 4
         return int(self._plan_ws[lo:lo + self.plan.stage_item[32]].sum())
+
+    def items_per_partition(self):
+        """Work items each partition is split into (per lane group); a run's
+        part_cycles is their sum."""
+        if self.plan is None:
+            return np.ones(self.num_partitions, np.int64)
+        ws, n = self._plan_ws, self.plan.stage_item[32]
+        lo = (self.plan.item_off - ws.data_ptr()) // 4
+        off = ws[lo:lo + 2 * n].view(torch.int64)
+        part = ws[(self.plan.blob - ws.data_ptr()) // 4 + off + PLAN_ITEM_PARTITION]
+        return np.bincount(part.cpu().numpy(), minlength=self.num_partitions)
 
     def octet_need(self):
         """The most 64-byte tree slots an octet item needs for any partition

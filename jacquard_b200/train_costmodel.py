@@ -10,7 +10,8 @@
    per item, the batched workload's form; --per-item 2 for lane pairs) with
    per-partition timing (`part_cycles`, which leaves out the grid-barrier
    wait) and records log(mean SM cycles per work item) next to the
-   partition's 24 features.
+   partition's 24 features (a partition that the plan splits counts as the
+   mean of its items, which run side by side).
 3. Trains the MLP with Adam (lr 1e-3, batch 512) on the GPU kernels.
 4. Evaluates on fresh designs: balanced partitions without and with the
    learned cut choice (each major stage is cut with several weights of a
@@ -50,7 +51,8 @@ def measure(design, split_every, parts, lanes=8, cycles=4, blocks=148, per_item=
     B.run(None, cycles, part_cycles=pc)
     torch.cuda.synchronize()
     assert B.status() == 0
-    t_item = pc.cpu().numpy().astype(np.float64) / ((lanes // per_item) * cycles)
+    items = np.maximum(1, B.items_per_partition())
+    t_item = pc.cpu().numpy().astype(np.float64) / ((lanes // per_item) * cycles * items)
     ok = t_item > 0
     return s.features[ok], np.log(t_item[ok]).astype(np.float32)
 

@@ -379,3 +379,27 @@ def test_planned_octets_do_not_keep_the_prepared_script():
     assert B.plan is not None and B._prep is None
     assert B.prepared.numel() == B.ds.blocks_data.numel()
     assert B.octet_need() <= batched.octet_capacity()
+
+
+@pytest.mark.parametrize("parts,split_into", [(37, 4), (148, 1)])
+def test_items_of_split_partitions(parts, split_into):
+    """Octet items of the training family: every partition of a full stage in
+    as many items as fill the SMs, and part_cycles their sum."""
+    s = cases.script("soc_mini", 148, (20, 40, 60), xprop=True, target_parts=parts)
+    B = batched.BatchedSim(s, 8, lanes_per_item=0)
+    per = B.items_per_partition()
+    stage = np.asarray(s.stage_block_part)[:, 0]
+    assert per.sum() == B.plan.stage_item[32] and per.min() >= 1
+    groups = 8 // B.plan.lanes_per_item
+    for ms in range(s.num_major_stages):
+        n = int((stage == ms).sum())
+        want = max(1, min(16, (148 // groups) // n))
+        assert (per[stage == ms] == want).all()
+    if B.plan.lanes_per_item == 8:
+        assert per.max() == split_into
+    pc = torch.zeros(s.num_partitions, dtype=torch.int64, device="cuda")
+    B.load_state(np.zeros((8, B.sig), np.uint32))
+    B.run(None, 3, part_cycles=pc)
+    assert B.status() == 0
+    assert (pc > 0).all()
+    assert (batched.BatchedSim(s, 8, lanes_per_item=0, planned=False).items_per_partition() == 1).all()
