@@ -59,16 +59,9 @@ KERNEL_SRC = os.path.join(HERE, "jacquard_b200", "csrc", "batched_plan.cuh")
 
 
 def kernel_code_hash(path=KERNEL_SRC):
-    """sha256 of a kernel source with its comments, trailing blanks and
-    empty lines removed: it changes with the code, not with comment edits."""
-    import hashlib
-    import re
-    with open(path) as f:
-        src = f.read()
-    src = re.sub(r"/\*.*?\*/", "", src, flags=re.S)
-    src = re.sub(r"//[^\n]*", "", src)
-    lines = [ln.rstrip() for ln in src.splitlines() if ln.strip()]
-    return hashlib.sha256("\n".join(lines).encode()).hexdigest()
+    """build.code_hash: it changes with the code, not with comment edits."""
+    from jacquard_b200 import build
+    return build.code_hash(path)
 
 
 def measured_traffic_per_cycle():
@@ -227,7 +220,7 @@ def learned_wins(parts_per_stage, lanes_per_item):
     streams) in the same configuration (partitions per major stage, lane
     words per work item), with the learned run bit-exact against the
     heuristic one.  The benchmark uses the learned cut by default only
-    then."""
+    then, and only while the kernel is the one it was measured on."""
     m = MODEL_PATHS.get(lanes_per_item)
     if m is None:
         return False
@@ -241,14 +234,29 @@ def learned_wins(parts_per_stage, lanes_per_item):
             and ev.get("lanes_per_item", 2) == lanes_per_item)
 
 
+def measured_on_this_kernel(lanes_per_item):
+    """Whether the summary learned_wins() reads was measured on the batched
+    kernel's present code (its "kernel" is a prefix of kernel_code_hash)."""
+    with open(os.path.splitext(MODEL_PATHS[lanes_per_item])[0] + ".json") as f:
+        k = json.load(f).get("kernel", "")
+    return len(k) >= 12 and kernel_code_hash().startswith(k)
+
+
+def use_learned(learned, split_every, parts_per_stage, lanes_per_item):
+    """Whether `--learned` takes the learned cut ("auto": when it was measured
+    to win on the kernel as it is)."""
+    return learned == "on" or (learned == "auto" and split_every == 4 and
+                               learned_wins(parts_per_stage, lanes_per_item) and
+                               measured_on_this_kernel(lanes_per_item))
+
+
 def default_batched_script(d, blocks=148, lanes=8, per_item=8, learned="auto", split_every=4,
                            input_weight16=0):
     """(script, lanes per item) exactly as the batched mode builds them with
     these options: balanced partitions, one round of work items per major
     stage, the learned cut when `learned` says so."""
     per_stage = blocks // max(1, lanes // per_item)
-    use = learned == "on" or (learned == "auto" and split_every == 4 and
-                              learned_wins(per_stage, per_item))
+    use = use_learned(learned, split_every, per_stage, per_item)
     return build_script(d, blocks, cost_model=learned_model(per_item) if use else None,
                         target_parts=per_stage, split_every=split_every,
                         input_weight16=input_weight16), per_item
@@ -522,9 +530,8 @@ def run_mine_batched(args, rank, world):
     per_item = args.per_item
     while True:
         per_stage = args.blocks // max(1, args.lanes // per_item)  # one round of items
-        use_learned = args.learned == "on" or (args.learned == "auto" and args.split == 4 and
-                                               learned_wins(per_stage, per_item))
-        model = learned_model(per_item) if use_learned else None
+        model = learned_model(per_item) if use_learned(args.learned, args.split, per_stage,
+                                                       per_item) else None
         s, _ = default_batched_script(d, args.blocks, args.lanes, per_item, args.learned,
                                       args.split, args.input_weight16)
         po_sig = state.po_positions(s, d)

@@ -7,7 +7,9 @@
                        reference tree when it is present)
 """
 import glob
+import hashlib
 import os
+import re
 import shutil
 import subprocess
 
@@ -15,6 +17,20 @@ from ._native import PKG_DIR, REPO_DIR
 
 CSRC = os.path.join(PKG_DIR, "csrc")
 NVCC_ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+
+
+BATCHED_KERNEL = os.path.join(CSRC, "batched_plan.cuh")
+
+
+def code_hash(path=BATCHED_KERNEL):
+    """sha256 of a kernel source with its comments, trailing blanks and
+    empty lines removed: it changes with the code, not with comment edits."""
+    with open(path) as f:
+        src = f.read()
+    src = re.sub(r"/\*.*?\*/", "", src, flags=re.S)
+    src = re.sub(r"//[^\n]*", "", src)
+    lines = [ln.rstrip() for ln in src.splitlines() if ln.strip()]
+    return hashlib.sha256("\n".join(lines).encode()).hexdigest()
 
 
 def _gxx():

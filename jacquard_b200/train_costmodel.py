@@ -29,6 +29,7 @@ import numpy as np
 import torch
 
 from . import batched, costmodel, frontend, state
+from . import build as build_lib
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -208,6 +209,7 @@ def main():
     ev_soc = evaluate(m.pack(), clusters=512, cycles=args.eval_cycles, seed=2, parts=soc_parts,
                       per_item=pi)
     summary = {"samples": int(len(y)), "steps": args.steps, "per_item": pi,
+               "kernel": build_lib.code_hash()[:16],
                "loss_start": hist[0][1],
                "loss_end": hist[-1][1], "heldout_mse": mse, "heldout_var": base,
                "heldout_r2": 1 - mse / base, "eval": ev, "eval_soc2m": ev_soc}
