@@ -2,6 +2,7 @@
 #include "plan_build.cuh"
 
 #include <algorithm>
+#include <exception>
 
 namespace jqk {
 
@@ -686,7 +687,7 @@ const uint32_t *PlanBuilder::unwritten() const {
   return ws + PlanLayout(num_blocks * nms, parts, 0, state_words).unwritten;
 }
 
-int PlanBuilder::scan(bool *ok) {
+int PlanBuilder::scan_lists(bool *ok) {
   *ok = false;
   const size_t entries = num_blocks * nms;
   const PlanLayout l0(entries, 0, 0, 0);
@@ -737,7 +738,8 @@ int PlanBuilder::scan(bool *ok) {
   return JQ_OK;
 }
 
-int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok) {
+int PlanBuilder::build_items(PlanMode mode, size_t want, size_t round, uint32_t pair_gates,
+                             bool *ok) {
   *ok = false;
   const size_t entries = num_blocks * nms;
   std::vector<uint32_t> items;
@@ -800,7 +802,7 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
   item_words = B.item_words;
   if ((r.unsupported & 4u) && split_srams) {  // once more without splitting those
     split_srams = false;
-    return build(mode, want, round, pair_gates, ok);
+    return build_items(mode, want, round, pair_gates, ok);
   }
   *ok = !r.unsupported;
   overflow = r.unsupported == 8u;
@@ -835,6 +837,24 @@ int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_g
       return JQ_ERR_CUDA;
   }
   return JQ_OK;
+}
+
+// The lists above are the only host allocations: a caller of the C interface
+// gets a status when there is no memory for them.
+int PlanBuilder::scan(bool *ok) {
+  try {
+    return scan_lists(ok);
+  } catch (const std::exception &) {
+    return JQ_ERR_INVALID_ARG;
+  }
+}
+
+int PlanBuilder::build(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok) {
+  try {
+    return build_items(mode, want, round, pair_gates, ok);
+  } catch (const std::exception &) {
+    return JQ_ERR_INVALID_ARG;
+  }
 }
 
 }  // namespace jqk

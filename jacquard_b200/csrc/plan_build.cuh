@@ -91,6 +91,10 @@ struct PlanBuilder {
   // by decreasing size, every second round reversed.  Items whose levels
   // average at most pair_gates gates list them by pair of levels.
   int build(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok);
+
+  // the work of the two; they throw when host memory runs out
+  int scan_lists(bool *ok);
+  int build_items(PlanMode mode, size_t want, size_t round, uint32_t pair_gates, bool *ok);
 };
 
 // Words of workspace a build of any script of this size fits in.

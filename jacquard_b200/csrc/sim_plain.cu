@@ -857,6 +857,8 @@ bool legacy_planned(const jq_sim_args *a, int *rc) {
   if (ok) {
     *rc = launch_planned(a, &plan, nullptr, nullptr, pc.ws + plan_words);
     if (*rc == JQ_OK) *rc = read_status(nullptr);
+  } else {
+    cudaGetLastError();  // the script's own launch starts clean
   }
   if (pc.words * 4 > LEGACY_PLAN_KEEP) {
     cudaFree(pc.ws);
