@@ -13,7 +13,8 @@ batched mode partitions every major stage into blocks / (lanes / per-item)
 balanced partitions: one round of work items, octet items (8 lane words,
 the default) or lane pairs.  With --learned the cost model trained on that
 item form chooses each stage's cut (auto: only when its committed training
-summary shows it winning, bit-exact, on this design in this configuration).
+summary shows it winning, bit-exact, on this design in this configuration and
+on the present kernel).
 `value` is device-timed throughput with inputs resident in HBM; `e2e` is the
 same through the C ABI with host buffers copied in and out inside the timed
 region; `parity` is the replay of two sampled streams of both timed regions
@@ -1015,7 +1016,8 @@ def main():
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--learned", default="auto", choices=["auto", "on", "off"],
                     help="batched / timed: the learned cost model chooses each stage's balanced "
-                         "cut (auto: when its recorded gain on this design is above 1)")
+                         "cut (auto: when its gain on this design, recorded on the "
+                         "present kernel, is above 1)")
     ap.add_argument("--no-check", action="store_true",
                     help="batched: skip the bit-exactness self-check of the timed windows")
     ap.add_argument("--no-compare", action="store_true",

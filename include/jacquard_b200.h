@@ -157,8 +157,9 @@ int jq_plain_prepare(const size_t *blocks_start, const uint32_t *blocks_data, si
  * partitions are split towards (0 = default; 0xffffffff = default, and never
  * the mirrored form).  `supported` is 0 for a script
  * that the plan does not represent: one whose partitions read writeout slots
- * that nothing in the partition writes, or words of their own major stage,
- * or that exceed its limits; jq_simulate runs those. */
+ * that nothing in the partition writes, words of their own major stage or X
+ * words as values, share an SRAM, or exceed its limits; jq_simulate runs
+ * those. */
 typedef struct {
   size_t num_blocks, num_major_stages;
   uint32_t supported;                   /* 0: not represented, run jq_simulate */

@@ -7,7 +7,7 @@
 // What bounds it: latency.  A major stage of one stream is a chain of state
 // word exchange, a few gate levels and the commit; an item's blob (up to
 // about 60 KB) is copied by TMA one item ahead.  us per pass, script form / plan:
-// 16k gates x 64 cycles 2722 / 537, 2M gates x 16 cycles 6130 / 1224, 256k
+// 16k gates x 64 cycles 2721 / 532, 2M gates x 16 cycles 5742 / 1156, 256k
 // gates x 32 cycles 4918 / 1486.
 #pragma once
 #include "plan_build.cuh"

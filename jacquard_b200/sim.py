@@ -84,7 +84,9 @@ def dev_to_u32(t):
 
 
 class DeviceScript:
-    """Script arrays resident on the device."""
+    """Script arrays resident on the device.  The plan, stage depths and
+    arrivals made from them on first use are kept: a changed script takes a new
+    DeviceScript."""
 
     def __init__(self, script, device="cuda"):
         self.script = script
